@@ -30,7 +30,7 @@
 #include <stdint.h>
 
 #include "rb200_internal.h"
-#include "stage_kernel.cuh"  // logavg, Mode
+#include "stage_kernel.cuh"  // log_mean, Mode
 
 namespace rb200 {
 
@@ -342,6 +342,7 @@ __global__ void __launch_bounds__(Q * Q * Q / NPT, (pipe_min_ctas<T, Q>()))
     constexpr bool kStageDq = sizeof(T) == 4;
     const uint32_t qbytes = NS * NP * sizeof(double);
     const T gm1 = (T)(A.gamma - 1.0), gam = (T)A.gamma;
+    [[maybe_unused]] const T ec_inv_2gm1 = T(1) / (T(2) * gm1);
 
     Cursor<BATCH> cur;  // meaningful in threads 0..9
     if (t == 0) {
@@ -490,13 +491,11 @@ __global__ void __launch_bounds__(Q * Q * Q / NPT, (pipe_min_ctas<T, Q>()))
                 ac[4] = fma(un, pv[5], ac[4]);
             } else {
                 const T ua0 = (o[1] + pv[1]) * T(0.5), ua1 = (o[2] + pv[2]) * T(0.5), ua2 = (o[3] + pv[3]) * T(0.5);
-                const T ra = (o[0] + pv[0]) * T(0.5);
-                const T ba = (o[4] + pv[4]) * T(0.5);
                 const T u2a = (o[5] + pv[5]) * T(0.5);
-                const T rlog = logavg(o[0], pv[0]);
-                const T blog = logavg(o[4], pv[4]);
-                const T pt = ra / (T(2) * ba);
-                const T cc = T(1) / ((T(2) * gm1) * blog) - u2a * T(0.5);
+                const T ir = T(1) / (o[0] + pv[0]), ib = T(1) / (o[4] + pv[4]);
+                const T rlog = log_mean(o[0], pv[0], ir);
+                const T pt = (T(0.5) * (o[0] + pv[0])) * ib;  // rho_avg / (2 b_avg)
+                const T cc = ec_inv_2gm1 * inverse_log_mean(o[4], pv[4], ib) - u2a * T(0.5);
                 const T un = (dir == 0 ? ua0 : dir == 1 ? ua1 : ua2) * sc;
                 const T uaa = ua0 * ua0 + ua1 * ua1 + ua2 * ua2;
                 const T f0 = rlog * un;

@@ -96,26 +96,8 @@ struct Prefetched {
     bool tables_ready = false;
 };
 
-__device__ __forceinline__ double dev_log(double x) { return log(x); }
-__device__ __forceinline__ float dev_log(float x) { return logf(x); }
 __device__ __forceinline__ double dev_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float dev_sqrt(float x) { return sqrtf(x); }
-
-// logavg (numericalfluxes.jl:9-22)
-template <typename T>
-__device__ __forceinline__ T logavg(T a, T b) {
-    const T zeta = a / b;
-    const T f = (zeta - T(1)) / (zeta + T(1));
-    const T u = f * f;
-    const T eps = sizeof(T) == 8 ? T(2.220446049250313e-16) : T(1.1920929e-07f);
-    T F;
-    if (u < eps) {
-        F = fma(u, fma(u, fma(u, fma(u, T(1) / T(9), T(1) / T(7)), T(1) / T(5)), T(1) / T(3)), T(1));
-    } else {
-        F = dev_log(zeta) / (T(2) * f);
-    }
-    return (a + b) / (T(2) * F);
-}
 
 // Buffers of the element being updated: the DGSEM handle takes them from StageArgs,
 // the serving loop from each solve's descriptor.
@@ -405,6 +387,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
     for (int s = 0; s < NS; ++s) acc[s] = T(0);
     const int dmask = A.dir_mask ? A.dir_mask : 7;  // DGSEM(; directions)
+    [[maybe_unused]] const T ec_inv_2gm1 = T(1) / (T(2) * (T)(A.gamma - 1.0));
 
 #pragma unroll
     for (int dir = 0; dir < DIM; ++dir) {
@@ -481,13 +464,11 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
                     }
                     const T b2 = aux[(DIM + 1) * NP + na];
                     const T uu2 = aux[(DIM + 2) * NP + na];
-                    const T ra = (own[0] + r2) * T(0.5);
-                    const T ba = (own[DIM + 1] + b2) * T(0.5);
                     const T u2a = (own[DIM + 2] + uu2) * T(0.5);
-                    const T rlog = logavg(own[0], r2);
-                    const T blog = logavg(own[DIM + 1], b2);
-                    const T pt = ra / (T(2) * ba);
-                    const T c = T(1) / ((T(2) * (T)(A.gamma - 1.0)) * blog) - u2a * T(0.5);
+                    const T ir = T(1) / (own[0] + r2), ib = T(1) / (own[DIM + 1] + b2);
+                    const T rlog = log_mean(own[0], r2, ir);
+                    const T pt = (T(0.5) * (own[0] + r2)) * ib;  // rho_avg / (2 b_avg)
+                    const T c = ec_inv_2gm1 * inverse_log_mean(own[DIM + 1], b2, ib) - u2a * T(0.5);
                     T un = ua[0] * G[0], uaa = ua[0] * ua[0];
 #pragma unroll
                     for (int d = 1; d < DIM; ++d) {

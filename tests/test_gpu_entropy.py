@@ -205,3 +205,33 @@ def test_snapshot_resume(rb, cuda_ok, precision, stepper):
     with pytest.raises(rb.RB200Error) as ei:
         rb.restore(other, snap, q2, s2)
     assert ei.value.status == 2
+
+
+@pytest.mark.parametrize("ratio", [1.0, 1 + 1e-9, 1.01, 1.21, 1.23, 3.0])
+@pytest.mark.parametrize("dim,nq,sflux,precision", [(2, 5, "rusanov", "fp64"), (3, 4, "rusanov", "fp64"), (3, 5, "ec", "fp64"),
+                                                    (3, 8, "rusanov", "fp64"), (2, 4, "rusanov", "fp32_bulk")])
+def test_log_mean_branches(rb, cuda_ok, dim, nq, sflux, precision, ratio):
+    """The entropy-conservative tendency of states whose density and rho/p take two values
+    with a fixed ratio: equal values, values in the power series of the logarithmic mean and
+    of the reference (1 + 1e-9: both use a series), and both sides of the series' end (f =
+    0.1, a ratio of 1.222).  The bound is relative to the size of the summed terms,
+    2/h max_i sum_a |D[a,i] w_a/w_i - D[i,a]| max |flux| per field: 1e-12 in FP64, and 5e-6
+    (some 40 roundings of 2^-24) in FP32 bulk."""
+    og, dg, olaw, law = _build(rb, dim, nq, (3,) * dim, (1,) * dim, "eul_ec", O.WARP_NONE, sflux, precision)
+    rng = np.random.default_rng(5)
+    shape = (og.np, og.E)
+    rho = np.where(rng.random(shape) < 0.5, 1.0, ratio)
+    p = rho / np.where(rng.random(shape) < 0.5, 1.1, 1.1 * ratio)
+    u = [np.full(shape, v) for v in (0.4, -0.3, 0.2)[:dim]]
+    E = p / 0.4 + rho * sum(v * v for v in u) / 2
+    q = np.asfortranarray(np.stack([rho] + [rho * v for v in u] + [E], axis=1))
+    ref = og.tendency(olaw, q)
+    qg = rb.GridArray.from_numpy(q)
+    dqg = qg.similar()
+    dg(dqg, qg, 0.0, increment=False)
+    err = np.abs(dqg.numpy() - ref).max(axis=(0, 2))
+    _, w, D = og.lgl()
+    S = np.abs(D * (w[:, None] / w[None, :]) - D.T).sum(axis=0).max() * 2 / (10.0 / 3)
+    c = max(abs(v[0, 0]) for v in u)
+    scale = S * np.array([(rho * c).max()] + [(rho * c * c + p).max()] * dim + [((E + p) * c).max()])
+    assert (err <= (1e-12 if precision == "fp64" else 5e-6) * scale).all(), (err / scale)
