@@ -40,6 +40,8 @@ def _sources():
     for d in (2, 3):
         units.append((os.path.join(CSRC, "serve_inst.cu"), os.path.join(BUILD, f"serve_d{d}.o"),
                       [f"-DRB_SERVE_DIM={d}"]))
+    for q in range(4, 9):
+        units.append((os.path.join(CSRC, "line_inst.cu"), os.path.join(BUILD, f"line_q{q}.o"), [f"-DRB_LINE_NQ={q}"]))
     for name in ("dispatch", "reduce", "pipelined_inst", "serve", "utilities", "mortar", "relaxation", "diagnostics",
                  "halo", "api"):
         units.append((os.path.join(CSRC, f"{name}.cu"), os.path.join(BUILD, f"{name}.o"), []))

@@ -75,7 +75,7 @@ struct rb200_handle {
     int use_graphs = 1;
     int pipe_grid = 0;            // CTAs of the pipelined kernel (0: not eligible)
     int pipe_curved_grid = 0;     // CTAs of the curved-grid pipelined kernel, FP32 bulk or FP64 (0: not eligible)
-    double pipe_S[64] = {0};      // D[a,id] w[a] / w[id] - D[id,a] (advection: D[a,id] w[a] / w[id])
+    PipeArgs pipe{};              // its tables and constants; a launch adds its buffers and coefficients
     // mortars of an adapted grid (rb200_set_mortars)
     int64_t nmortars = 0;
     int64_t* d_mortars = nullptr;
@@ -246,8 +246,7 @@ cudaError_t launch_any(rb200_handle* h, const StageArgs& a, cudaStream_t st) {
                           (!stage_mode || aligned16(a.q_out)) &&
                           (h->prec == RB200_PRECISION_FP64 || stage_mode);
     if (!eligible) return launch_stage(h->dim, h->nq, h->combo, h->geom, h->prec, a, st);
-    PipeArgs p;
-    std::memset(&p, 0, sizeof(p));
+    PipeArgs p = h->pipe;
     p.q_in = a.q_in;
     p.q_out = a.q_out;
     p.dq = a.dq;
@@ -261,11 +260,6 @@ cudaError_t launch_any(rb200_handle* h, const StageArgs& a, cudaStream_t st) {
     p.surface_rusanov = a.surface_rusanov;
     p.rka = a.rka;
     p.rkb_dt = a.rkb_dt;
-    p.gamma = a.gamma;
-    std::memcpy(p.S, h->pipe_S, sizeof(p.S));
-    for (int i = 0; i < 64; ++i) p.Sf[i] = (float)h->pipe_S[i];
-    std::memcpy(p.w, h->w, sizeof(p.w));
-    std::memcpy(p.adv, a.adv, sizeof(p.adv));
     const int grid = (int)std::min<int64_t>(h->pipe_grid, a.E - a.e_begin);
     return launch_pipelined(h->nq, h->combo, h->prec, p, grid, st);
 }
@@ -765,15 +759,12 @@ rb200_status rb200_create(const rb200_desc* d, rb200_handle** out) {
     if ((st = dev_alloc(h, &h->d_status, 1)) != RB200_OK) return bail(st);
     ce = cudaMemset(h->d_status, 0, sizeof(int32_t));
     if (ce != cudaSuccess) return bail(cuda_fail(h, ce, "memset"));
-    if (dim == 3 && (nq == 4 || nq == 6 || nq == 8) && affine &&
-        (h->combo == EUL_KG || h->combo == EUL_EC || h->combo == ADV_WEAK) && !entropy_flux) {
-        // flux differencing: S[a, id] = D[a,id] w[a] / w[id] - D[id,a]; weak-form
-        // advection: W[a, id] = D[a,id] w[a] / w[id]
-        for (int a = 0; a < nq; ++a)
-            for (int id = 0; id < nq; ++id)
-                h->pipe_S[a * nq + id] = h->combo == ADV_WEAK
-                                             ? h->D[a + nq * id] * (h->w[a] / h->w[id])
-                                             : h->D[a + nq * id] * (h->w[a] / h->w[id]) - h->D[id + nq * a];
+    // 3-D bricks: the half-line kernel (Euler, Nq = 4..8) or the advection kernel (Nq = 4, 6, 8)
+    const bool adv_pipe = h->combo == ADV_WEAK && (nq == 4 || nq == 6 || nq == 8);
+    const bool line_pipe = h->law == RB200_LAW_EULER && nq >= 4 && !entropy_flux;
+    if (dim == 3 && affine && (adv_pipe || line_pipe) &&
+        (pipe_tables(h->pipe, h->combo, nq, h->gamma, h->D, h->w) || adv_pipe)) {
+        for (int d = 0; d < 3; ++d) h->pipe.adv[d] = h->adv[d];
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

@@ -46,7 +46,7 @@ constexpr int NT = 256, NVG = 11;
 
 struct Smem {
     double q[NS][NP];                 // element state (bulk copy)
-    pipe::AuxBuf<double> aux;         // partner values
+    pipe::Partners<double, NPP, 0> aux;         // partner values
     double2 lga[3][NPP];              // l_g[dir][0..1] of each node
     double lgb[3][NPP];               // l_g[dir][2]
     double slot[NS][NSLOT];           // neighbour trace, then (wsJ nf) MJI per face slot
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256, 2) pipelined_curved64_kernel(const __grid
             own[h][3] = m2 * rinv * 0.5;
             own[h][4] = rhoe * rinv * 0.5;
             own[h][5] = p * 0.5;
-            sm.aux.put(PAD(n), own[h]);
+            sm.aux.put(PAD(n), 0, own[h]);
 #pragma unroll
             for (int dir = 0; dir < 3; ++dir) {
                 sm.lga[dir][PAD(n)] = make_double2(vgl[h][3 * dir], vgl[h][3 * dir + 1]);
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256, 2) pipelined_curved64_kernel(const __grid
                     const int kk = k0 + 4 * h;
                     const int na = dir == 0 ? a + 8 * (jj + 8 * kk) : ii + 8 * (a + 8 * kk);
                     double pv[NAUX];
-                    sm.aux.get(PAD(na), pv);
+                    sm.aux.get(PAD(na), 0, pv);
                     pair(acc[h], own[h], pv, sm.lga[dir][PAD(na)], sm.lgb[dir][PAD(na)], lo[h], Dai, Dia);
                 }
             }
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256, 2) pipelined_curved64_kernel(const __grid
             for (int a = 0; a < NQ; ++a) {
                 const int nz = ii + 8 * (jj + 8 * a);
                 double pv[NAUX];
-                sm.aux.get(PAD(nz), pv);
+                sm.aux.get(PAD(nz), 0, pv);
                 const double2 la = sm.lga[2][PAD(nz)];
                 const double lb = sm.lgb[2][PAD(nz)];
 #pragma unroll
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(256, 2) pipelined_curved64_kernel(const __grid
             double qm[NS], qp[NS], Fm[NS], Fp[NS], wm, wp;
             {
                 double v[NAUX];
-                sm.aux.get(PAD(vn), v);
+                sm.aux.get(PAD(vn), 0, v);
                 const double rho = 2.0 * v[0];
                 qm[0] = rho;
                 qm[1] = rho * (2.0 * v[1]);

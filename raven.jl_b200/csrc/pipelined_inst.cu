@@ -1,6 +1,6 @@
-// Instantiations and launch helpers of the pipelined 3-D stage kernels (Euler flux
-// differencing and weak-form advection, Nq = 4, 6, 8): one state (the DGSEM handle) or
-// the chunks of a serving class (BATCH).
+// Instantiations and launch helpers of the pipelined 3-D stage kernels: Euler on bricks (the
+// half-line kernel of line_inst.cu), weak-form advection on bricks and curved grids; one
+// state (the DGSEM handle) or the chunks of a serving class (BATCH).
 #include "pipelined_adv.cuh"
 #include "pipelined_curved.cuh"
 #include "pipelined_curved64.cuh"
@@ -8,17 +8,22 @@
 
 namespace rb200 {
 
-template <int COMBO, typename T, bool BATCH, int Q>
-static cudaError_t launch_p(const PipeArgs& a, const PipeBatch& b, int grid, cudaStream_t s) {
-    constexpr int kNPT = pipe_npt<T, Q>();
-    auto kern = pipelined_stage_kernel<COMBO, T, kNPT, BATCH, Q>;
-    static std::atomic<uint64_t> configured{0};
-    cudaError_t err = ensure_smem_limit(kern, (int)sizeof(pipe::Smem<T, Q>), configured);
-    if (err != cudaSuccess) return err;
-    if constexpr (!BATCH)  // serving ticks follow host-written chunk tables: plain order
-        return launch_pdl(kern, grid, Q * Q * Q / kNPT, sizeof(pipe::Smem<T, Q>), s, a, b);
-    kern<<<grid, Q * Q * Q / kNPT, sizeof(pipe::Smem<T, Q>), s>>>(a, b);
-    return cudaGetLastError();
+#define RB_LINE_DECL(Q)                                                                                            \
+    cudaError_t launch_line_q##Q(int combo, int fp32, bool batch, const PipeArgs& a, const PipeBatch& b, int grid, \
+                                 cudaStream_t s, int* blocks_per_sm);
+RB_LINE_DECL(4) RB_LINE_DECL(5) RB_LINE_DECL(6) RB_LINE_DECL(7) RB_LINE_DECL(8)
+
+// The Euler law: the half-line kernel (line_inst.cu).
+static cudaError_t launch_line(int nq, int combo, int fp32, bool batch, const PipeArgs& a, const PipeBatch& b, int grid,
+                               cudaStream_t s, int* bps) {
+    switch (nq) {
+        case 4: return launch_line_q4(combo, fp32, batch, a, b, grid, s, bps);
+        case 5: return launch_line_q5(combo, fp32, batch, a, b, grid, s, bps);
+        case 6: return launch_line_q6(combo, fp32, batch, a, b, grid, s, bps);
+        case 7: return launch_line_q7(combo, fp32, batch, a, b, grid, s, bps);
+        case 8: return launch_line_q8(combo, fp32, batch, a, b, grid, s, bps);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 // The advection law: one field, pipea::npt<Q>() nodes a thread.
@@ -32,60 +37,26 @@ static cudaError_t launch_a(const PipeArgs& a, const PipeBatch& b, int grid, cud
     return cudaGetLastError();
 }
 
-template <int COMBO, typename T, bool BATCH>
-static cudaError_t launch_q(int nq, const PipeArgs& a, const PipeBatch& b, int grid, cudaStream_t s) {
-    if constexpr (COMBO == ADV_WEAK) {
-        switch (nq) {
-            case 4: return launch_a<T, BATCH, 4>(a, b, grid, s);
-            case 6: return launch_a<T, BATCH, 6>(a, b, grid, s);
-            case 8: return launch_a<T, BATCH, 8>(a, b, grid, s);
-            default: return cudaErrorInvalidValue;
-        }
-    }
+template <typename T, bool BATCH>
+static cudaError_t launch_adv(int nq, const PipeArgs& a, const PipeBatch& b, int grid, cudaStream_t s) {
     switch (nq) {
-        case 4: return launch_p<COMBO, T, BATCH, 4>(a, b, grid, s);
-        case 6: return launch_p<COMBO, T, BATCH, 6>(a, b, grid, s);
-        case 8: return launch_p<COMBO, T, BATCH, 8>(a, b, grid, s);
+        case 4: return launch_a<T, BATCH, 4>(a, b, grid, s);
+        case 6: return launch_a<T, BATCH, 6>(a, b, grid, s);
+        case 8: return launch_a<T, BATCH, 8>(a, b, grid, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_pipelined(int nq, int combo, int fp32, const PipeArgs& a, int grid, cudaStream_t s) {
     const PipeBatch none{};
-    if (combo == EUL_KG)
-        return fp32 ? launch_q<EUL_KG, float, false>(nq, a, none, grid, s)
-                    : launch_q<EUL_KG, double, false>(nq, a, none, grid, s);
-    if (combo == EUL_EC)
-        return fp32 ? launch_q<EUL_EC, float, false>(nq, a, none, grid, s)
-                    : launch_q<EUL_EC, double, false>(nq, a, none, grid, s);
-    if (combo == ADV_WEAK)
-        return fp32 ? launch_q<ADV_WEAK, float, false>(nq, a, none, grid, s)
-                    : launch_q<ADV_WEAK, double, false>(nq, a, none, grid, s);
-    return cudaErrorInvalidValue;
+    if (combo != ADV_WEAK) return launch_line(nq, combo, fp32, false, a, none, grid, s, nullptr);
+    return fp32 ? launch_adv<float, false>(nq, a, none, grid, s) : launch_adv<double, false>(nq, a, none, grid, s);
 }
 
 cudaError_t launch_pipelined_batch(int nq, int combo, int fp32, const PipeArgs& a, const PipeBatch& b, int grid,
                                    cudaStream_t s) {
-    if (combo == EUL_KG)
-        return fp32 ? launch_q<EUL_KG, float, true>(nq, a, b, grid, s) : launch_q<EUL_KG, double, true>(nq, a, b, grid, s);
-    if (combo == ADV_WEAK)
-        return fp32 ? launch_q<ADV_WEAK, float, true>(nq, a, b, grid, s)
-                    : launch_q<ADV_WEAK, double, true>(nq, a, b, grid, s);
-    return cudaErrorInvalidValue;
-}
-
-template <int COMBO, typename T, bool BATCH, int Q>
-static int occupancy_p() {
-    constexpr int kNPT = pipe_npt<T, Q>();
-    auto kern = pipelined_stage_kernel<COMBO, T, kNPT, BATCH, Q>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(pipe::Smem<T, Q>)) !=
-        cudaSuccess)
-        return 0;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, Q * Q * Q / kNPT, sizeof(pipe::Smem<T, Q>)) !=
-        cudaSuccess)
-        return 0;
-    return n;
+    if (combo != ADV_WEAK) return launch_line(nq, combo, fp32, true, a, b, grid, s, nullptr);
+    return fp32 ? launch_adv<float, true>(nq, a, b, grid, s) : launch_adv<double, true>(nq, a, b, grid, s);
 }
 
 template <typename T, bool BATCH, int Q>
@@ -101,37 +72,29 @@ static int occupancy_a() {
     return n;
 }
 
-template <int COMBO, typename T, bool BATCH>
-static int occupancy_q(int nq) {
-    if constexpr (COMBO == ADV_WEAK) {
-        switch (nq) {
-            case 4: return occupancy_a<T, BATCH, 4>();
-            case 6: return occupancy_a<T, BATCH, 6>();
-            case 8: return occupancy_a<T, BATCH, 8>();
-            default: return 0;
-        }
-    }
+template <typename T, bool BATCH>
+static int occupancy_adv(int nq) {
     switch (nq) {
-        case 4: return occupancy_p<COMBO, T, BATCH, 4>();
-        case 6: return occupancy_p<COMBO, T, BATCH, 6>();
-        case 8: return occupancy_p<COMBO, T, BATCH, 8>();
+        case 4: return occupancy_a<T, BATCH, 4>();
+        case 6: return occupancy_a<T, BATCH, 6>();
+        case 8: return occupancy_a<T, BATCH, 8>();
         default: return 0;
     }
 }
 
+static int occupancy_line(int nq, int combo, int fp32, bool batch) {
+    int n = 0;
+    return launch_line(nq, combo, fp32, batch, PipeArgs{}, PipeBatch{}, 0, nullptr, &n) == cudaSuccess ? n : 0;
+}
+
 int pipelined_blocks_per_sm(int nq, int combo, int fp32) {
-    if (combo == EUL_KG) return fp32 ? occupancy_q<EUL_KG, float, false>(nq) : occupancy_q<EUL_KG, double, false>(nq);
-    if (combo == EUL_EC) return fp32 ? occupancy_q<EUL_EC, float, false>(nq) : occupancy_q<EUL_EC, double, false>(nq);
-    if (combo == ADV_WEAK)
-        return fp32 ? occupancy_q<ADV_WEAK, float, false>(nq) : occupancy_q<ADV_WEAK, double, false>(nq);
-    return 0;
+    if (combo != ADV_WEAK) return occupancy_line(nq, combo, fp32, false);
+    return fp32 ? occupancy_adv<float, false>(nq) : occupancy_adv<double, false>(nq);
 }
 
 int pipelined_batch_blocks_per_sm(int nq, int combo, int fp32) {
-    if (combo == EUL_KG) return fp32 ? occupancy_q<EUL_KG, float, true>(nq) : occupancy_q<EUL_KG, double, true>(nq);
-    if (combo == ADV_WEAK)
-        return fp32 ? occupancy_q<ADV_WEAK, float, true>(nq) : occupancy_q<ADV_WEAK, double, true>(nq);
-    return 0;
+    if (combo != ADV_WEAK) return occupancy_line(nq, combo, fp32, true);
+    return fp32 ? occupancy_adv<float, true>(nq) : occupancy_adv<double, true>(nq);
 }
 
 // The curved-grid kernel (FP32 bulk, Kennedy-Gruber): two CTAs per SM.

@@ -319,26 +319,18 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
     c.chunk_elems = 8 * c.epb[1];
     int nsm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device);
-    c.pipelined = c.dim == 3 && (c.nq == 4 || c.nq == 6 || c.nq == 8) && (c.combo == EUL_KG || c.combo == ADV_WEAK);
+    PipeArgs pa{};
+    c.pipelined = c.dim == 3 && (c.nq == 4 || c.nq == 6 || c.nq == 8) && (c.combo == EUL_KG || c.combo == ADV_WEAK) &&
+                  (pipe_tables(pa, c.combo, c.nq, c.base.gamma, c.base.D, c.base.w) || c.combo == ADV_WEAK);
     if (c.pipelined) {
         // one configuration (the persistent TMA-pipelined kernel): nothing to tune
         c.ntiles = 1;
         c.tile = 0;
         const int bps = pipelined_batch_blocks_per_sm(c.nq, c.combo, c.prec);
         if (bps <= 0) return cudaErrorInvalidConfiguration;
-        PipeArgs pa{};
         pa.status = c.d_status;
         pa.surface_rusanov = c.base.surface_rusanov;
-        pa.gamma = c.base.gamma;
-        const int q = c.nq;
-        for (int a = 0; a < q; ++a)
-            for (int id = 0; id < q; ++id)
-                pa.S[a * q + id] = c.combo == ADV_WEAK
-                                       ? c.base.D[a + q * id] * (c.base.w[a] / c.base.w[id])
-                                       : c.base.D[a + q * id] * (c.base.w[a] / c.base.w[id]) - c.base.D[id + q * a];
-        for (int i = 0; i < q; ++i) pa.w[i] = c.base.w[i];
         for (int d = 0; d < 3; ++d) pa.adv[d] = c.base.adv[d];
-        for (int i = 0; i < 64; ++i) pa.Sf[i] = (float)pa.S[i];
         cudaGraph_t g = nullptr;
         e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;

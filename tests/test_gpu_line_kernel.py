@@ -1,0 +1,100 @@
+"""The half-line stage kernel of 3-D Euler on unwarped bricks (Nq = 4..8; Kennedy-Gruber,
+entropy conservative, central flux differencing and the weak form) against the oracle and
+the generic stage kernel: grids with fewer and with more elements than its CTAs, faces on
+the boundary, tendencies that set and that add, and buffers aligned to 16 bytes only.
+
+Tolerances, those of the other pipelined kernels: max |gpu - oracle| <= 1e-12 of max |oracle|
+per array in FP64 (the register after steps, a small difference of larger terms, 1e-11),
+1e-6 for the state after two FP32-bulk steps.
+"""
+
+import numpy as np
+import pytest
+
+import oracle as O
+from gpu_util import initial_state, oracle_law, product_scheme, rel_err, wrap_oracle_grid
+
+pytestmark = pytest.mark.gpu
+
+SCHEMES = ["eul_kg", "eul_ec", "eul_weak", "eul_fdc"]
+# more elements than CTAs (FP64: 12, 6, 4, 3, 2 an SM at Nq = 4..8)
+MANY = {4: (13, 12, 12), 5: (10, 10, 9), 6: (9, 9, 8), 7: (8, 8, 7), 8: (7, 7, 7)}
+
+
+def _build(rb, nq, K, per, scheme, precision="fp64"):
+    og = O.Grid(3, nq, K, [0.0] * 3, [10.0, 8.0, 9.0], per)
+    law, form = product_scheme(rb, scheme, 3)
+    dg = rb.DGSEM(law=law, grid=wrap_oracle_grid(og), volume_form=form, surface_numericalflux=rb.RusanovFlux(),
+                  precision=precision)
+    assert dg.pipelined_ctas > 0
+    return og, dg, oracle_law(scheme, 3)
+
+
+@pytest.mark.parametrize("nq", range(4, 9))
+@pytest.mark.parametrize("scheme", SCHEMES)
+def test_small_open_grid(rb, cuda_ok, scheme, nq):
+    """Both tendency modes against the oracle, and two steps against the generic kernel."""
+    og, dg, olaw = _build(rb, nq, (3, 2, 2), (1, 0, 1), scheme)
+    q = initial_state(og, olaw, scheme, seed=3)
+    ref = og.tendency(olaw, q)
+    qg, dq = rb.GridArray.from_numpy(q), rb.GridArray.from_numpy(q)
+    dg(dq, qg, 0.0, increment=False)
+    assert rel_err(dq.numpy(), ref) <= 1e-12
+    dq = rb.GridArray.from_numpy(q)
+    dg(dq, qg, 0.0, increment=True)
+    assert rel_err(dq.numpy(), ref + q) <= 1e-12
+    out = []
+    for path in ("auto", "generic"):
+        dg.set_kernel_path(path)
+        qs = rb.GridArray.from_numpy(q)
+        rb.LSRK54(dg, qs, 1e-3).dostep(qs, 2)
+        out.append(qs.numpy())
+    dg.set_kernel_path("auto")
+    dg.sync_status()
+    assert rel_err(out[0], out[1]) <= 1e-12
+
+
+@pytest.mark.parametrize("nq", range(4, 9))
+@pytest.mark.parametrize("scheme", ["eul_kg", "eul_weak"])
+def test_more_elements_than_ctas(rb, cuda_ok, scheme, nq):
+    og, dg, olaw = _build(rb, nq, MANY[nq], (1, 1, 1), scheme)
+    assert og.E > dg.pipelined_ctas
+    q = initial_state(og, olaw, scheme, seed=4)
+    qo, dqo = q.copy(order="F"), og.state(olaw)
+    for i in range(2):
+        og.lsrk54_step(olaw, qo, dqo, i * 1e-3, 1e-3)
+    qg = rb.GridArray.from_numpy(q)
+    s = rb.LSRK54(dg, qg, 1e-3)
+    s.dostep(qg, 2)
+    dg.sync_status()
+    assert rel_err(qg.numpy(), qo) <= 1e-12
+    assert rel_err(s.dq.numpy(), dqo) <= 1e-11
+    _, dg32, _ = _build(rb, nq, MANY[nq], (1, 1, 1), scheme, "fp32_bulk")
+    qg = rb.GridArray.from_numpy(q)
+    rb.LSRK54(dg32, qg, 1e-3).dostep(qg, 2)
+    dg32.sync_status()
+    assert rel_err(qg.numpy(), qo) <= 1e-6
+
+
+@pytest.mark.parametrize("nq", [5, 8])
+def test_sixteen_byte_alignment(rb, cuda_ok, nq):
+    """Buffers that start 16 bytes past a 32-byte boundary: the same bits as aligned ones."""
+    import torch
+
+    og, dg, olaw = _build(rb, nq, (3, 3, 2), (1, 1, 1), "eul_kg")
+    q = initial_state(og, olaw, "eul_kg", seed=5)
+    aligned = rb.GridArray.from_numpy(q)
+
+    def shifted(t):
+        s = torch.empty(t.numel() + 2, dtype=t.dtype, device=t.device)[2:].view(t.shape)
+        assert s.data_ptr() % 32 == 16
+        return rb.GridArray(s.copy_(t), aligned.ns, aligned.np, aligned.E)
+
+    moved = shifted(aligned.data)
+    a, b = rb.LSRK54(dg, aligned, 1e-3), rb.LSRK54(dg, moved, 1e-3)
+    b.dq = shifted(a.dq.data)
+    a.dostep(aligned, 1)
+    b.dostep(moved, 1)
+    dg.sync_status()
+    assert torch.equal(aligned.data, moved.data) and torch.equal(a.dq.data, b.dq.data)
+    assert np.isfinite(aligned.numpy()).all()
