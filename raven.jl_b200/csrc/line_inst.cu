@@ -23,8 +23,9 @@ cudaError_t launch_m(const PipeArgs& a, const PipeBatch& b, int grid, cudaStream
     if (err != cudaSuccess) return err;
     if (blocks_per_sm)  // occupancy query only
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, line::Shape<Q>::TH, smem);
-    if constexpr (!BATCH)  // serving ticks follow host-written chunk tables: plain order
-        return launch_pdl(kern, grid, line::Shape<Q>::TH, smem, s, a, b);
+    // a tick's first stage follows host-written chunk tables: plain order; its others read what
+    // that stage has read, and wait for the stage before them like a single state's
+    if (!BATCH || b.stage > 0) return launch_pdl(kern, grid, line::Shape<Q>::TH, smem, s, a, b);
     kern<<<grid, line::Shape<Q>::TH, smem, s>>>(a, b);
     return cudaGetLastError();
 }

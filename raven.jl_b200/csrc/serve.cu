@@ -20,6 +20,7 @@
 //
 // A host thread runs the loop, and nothing on the device waits on the host.
 #include <cuda_runtime.h>
+#include <sys/prctl.h>
 
 #include <algorithm>
 #include <chrono>
@@ -103,7 +104,8 @@ const double kRKB[5] = {1432997174477.0 / 9575080441755.0, 5161836677717.0 / 136
                         2277821191437.0 / 14882151754819.0};
 
 constexpr int kMaxSolvesPerClass = 1024;
-constexpr int kMaxChunksPerClass = 1 << 16;
+constexpr int kMaxChunksPerClass = 1 << 16;  // at chunk_elems each
+constexpr int kMaxTableChunks = kMaxChunksPerClass + (1 << 14);  // and in the table: see launch_ticks
 constexpr size_t kAlign = 256;
 
 double now_s() {
@@ -207,8 +209,11 @@ struct Class {
     std::vector<SolveDesc> h_solves;
     std::vector<Chunk> h_chunks;
     std::vector<Solve*> slots;
-    int chunk_elems = 1;
-    int nchunks = 0;
+    int chunk_elems = 1;                         // elements of a chunk at most; admission counts these
+    int tile_elems = 1;                          // and at least
+    int grid = 1;                                // CTAs of the class's launches
+    int nchunks = 0;                             // chunks of the running solves at chunk_elems each
+    int32_t table_chunks = 0;                    // chunks in the table (upload source)
     int64_t tick = 0;
     bool dirty = true;
     int ntiles = 0;
@@ -219,11 +224,13 @@ struct Class {
     double tune_ms[3] = {0, 0, 0};
     int tune_n[3] = {0, 0, 0};
     int last_tile = 1;
+    int in_flight = 0;                           // ticks enqueued and not yet finished
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // tick start and end
     // totals of the completed ticks: device time between the tick's events (classes run
     // concurrently, so these overlap across classes) and DOF updates
     int64_t ticks_done = 0;
     double busy_ms = 0.0, dof_updates = 0.0;
+    double last_ms = 0.0;                        // device time of one of the last ticks
     bool pipelined = false;                      // 3-D Nq=4, 6, 8 Euler KG or advection: the pipelined kernel
     int32_t* d_status = nullptr;                 // its bounded waits report here
     int active = 0;
@@ -299,11 +306,11 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
     std::memcpy(c.base.D, r.D, sizeof(c.base.D));
     std::memcpy(c.base.w, r.w, sizeof(c.base.w));
     c.h_solves.assign(kMaxSolvesPerClass, SolveDesc{});
-    c.h_chunks.assign(kMaxChunksPerClass, Chunk{-1, 0, 0});
+    c.h_chunks.assign(kMaxTableChunks, Chunk{-1, 0, 0});
     c.slots.assign(kMaxSolvesPerClass, nullptr);
     cudaError_t e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c.d_solves, sizeof(SolveDesc) * kMaxSolvesPerClass);
-    if (e == cudaSuccess) e = cudaMalloc(&c.d_chunks, sizeof(Chunk) * kMaxChunksPerClass);
+    if (e == cudaSuccess) e = cudaMalloc(&c.d_chunks, sizeof(Chunk) * kMaxTableChunks);
     if (e == cudaSuccess) e = cudaMalloc(&c.d_nchunks, sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc(&c.d_tick, sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(c.d_nchunks, 0, sizeof(int32_t), c.stream);
@@ -328,6 +335,7 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
         c.tile = 0;
         const int bps = pipelined_batch_blocks_per_sm(c.nq, c.combo, c.prec);
         if (bps <= 0) return cudaErrorInvalidConfiguration;
+        c.grid = bps * nsm;
         pa.status = c.d_status;
         pa.surface_rusanov = c.base.surface_rusanov;
         for (int d = 0; d < 3; ++d) pa.adv[d] = c.base.adv[d];
@@ -357,6 +365,10 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
         e = launch_batched(c.dim, c.nq, c.combo, c.prec, t, probe, 0, c.stream, &bps);
         if (e != cudaSuccess) return e;
         const int grid = std::max(1, bps) * nsm;  // fixed persistent grid
+        if (t == 1 || c.ntiles == 1) {
+            c.grid = grid;
+            c.tile_elems = c.epb[1];
+        }
         cudaGraph_t g = nullptr;
         e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
@@ -444,7 +456,7 @@ cudaError_t admit(rb200_server* s) {
         d.nbr = reinterpret_cast<const int32_t*>(g + align_up((size_t)r->E * 4 * 8));
         d.E = r->E;
         d.dt = r->dt;
-        d.start_tick = c.tick + (c.launched ? 1 : 0);  // joins at the class's next tick
+        d.start_tick = c.tick + c.in_flight;  // joins at the class's next tick to be enqueued
         cudaError_t e = cudaMemcpyAsync(const_cast<double*>(d.elem_geo), r->geo.data(), r->geo.size() * 8,
                                         cudaMemcpyHostToDevice, s->upload);
         if (e == cudaSuccess)
@@ -495,48 +507,78 @@ cudaError_t admit(rb200_server* s) {
     return cudaSuccess;
 }
 
-cudaError_t launch_tick(Class& c) {
+// Enqueues the class's next ticks: one while the autotuner times them, else as many as run
+// before the first solve finishes, up to some kBatchMs of device time, so that a class of
+// small solves does not wait for the host between its ticks (a tick of a few small solves
+// takes 30-60 us of the device, the host's poll as long again).  A request that arrives
+// meanwhile joins behind them.
+//
+// A chunk is the work of one CTA at a time, so the table splits the running elements evenly:
+// about two chunks a CTA, of tile_elems to chunk_elems elements.  (At a fixed 8 tiles a 9^3
+// solve at Nq = 8 gave 92 of 444 CTAs 8 elements each.)  A table so has at most the chunks
+// that admission counted plus two for each CTA and one for each solve.
+constexpr double kBatchMs = 0.25;
+constexpr int kMaxBatch = 16;
+cudaError_t launch_ticks(Class& c) {
     cudaError_t e = cudaSuccess;
     if (c.dirty) {
+        int64_t total = 0;
+        for (int i = 0; i < kMaxSolvesPerClass; ++i)
+            if (c.slots[i]) total += c.h_solves[i].E;
+        const int64_t tiles = (total + 2 * (int64_t)c.grid * c.tile_elems - 1) / (2 * (int64_t)c.grid * c.tile_elems);
+        const int64_t len = std::min<int64_t>(std::max<int64_t>(tiles, 1) * c.tile_elems, c.chunk_elems);
         int n = 0;
         for (int i = 0; i < kMaxSolvesPerClass; ++i) {
             if (!c.slots[i]) continue;
             const int64_t E = c.h_solves[i].E;
-            for (int64_t f = 0; f < E; f += c.chunk_elems)
-                c.h_chunks[n++] = Chunk{i, (int32_t)std::min<int64_t>(c.chunk_elems, E - f), f};
+            for (int64_t f = 0; f < E && n < kMaxTableChunks; f += len)
+                c.h_chunks[n++] = Chunk{i, (int32_t)std::min<int64_t>(len, E - f), f};
         }
-        c.nchunks = n;
+        c.table_chunks = n;
         e = cudaMemcpyAsync(c.d_solves, c.h_solves.data(), sizeof(SolveDesc) * kMaxSolvesPerClass,
                             cudaMemcpyHostToDevice, c.stream);
         if (e == cudaSuccess && n)
             e = cudaMemcpyAsync(c.d_chunks, c.h_chunks.data(), sizeof(Chunk) * n, cudaMemcpyHostToDevice, c.stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(c.d_nchunks, &c.nchunks, sizeof(int32_t), cudaMemcpyHostToDevice, c.stream);
+            e = cudaMemcpyAsync(c.d_nchunks, &c.table_chunks, sizeof(int32_t), cudaMemcpyHostToDevice, c.stream);
         if (e != cudaSuccess) return e;
         c.dirty = false;
     }
     // autotuner: the first 2*ntiles ticks cycle through the tiles, then the fastest stays
     const bool tuning = c.tune_done < 2 * c.ntiles;
     c.last_tile = tuning ? c.tune_done % c.ntiles : c.tile;
+    int batch = 1;
+    if (!tuning) {
+        int64_t left = kMaxBatch;
+        for (auto* sv : c.slots)
+            if (sv) left = std::min<int64_t>(left, sv->req->nsteps - sv->steps_done);
+        const double ms = c.ticks_done > 0 ? c.last_ms : kBatchMs;
+        if (ms * left > kBatchMs) left = (int64_t)(kBatchMs / ms);
+        batch = (int)std::max<int64_t>(left, 1);
+    }
     e = cudaEventRecord(c.ev0, c.stream);
-    if (e == cudaSuccess) e = cudaGraphLaunch(c.graph[c.last_tile], c.stream);
-    if (e == cudaSuccess) e = cudaEventRecord(c.ev1, c.stream);  // completion of the tick
+    for (int k = 0; k < batch && e == cudaSuccess; ++k) e = cudaGraphLaunch(c.graph[c.last_tile], c.stream);
+    if (e == cudaSuccess) e = cudaEventRecord(c.ev1, c.stream);  // completion of the ticks
     c.launched = e == cudaSuccess;
+    c.in_flight = c.launched ? batch : 0;
     return e;
 }
 
-// After the class's tick completed on the device: bookkeeping; caller holds s->mu.
-cudaError_t finish_tick(rb200_server* s, Class& c) {
+// After the class's ticks completed on the device: bookkeeping; caller holds s->mu.
+cudaError_t finish_ticks(rb200_server* s, Class& c) {
+    const int batch = c.in_flight;
     c.launched = false;
-    const int64_t done_tick = c.tick;
+    c.in_flight = 0;
+    const int64_t done_tick = c.tick;  // the first of them
     float ms = 0;
     cudaEventElapsedTime(&ms, c.ev0, c.ev1);
-    int64_t elems = 0;  // elements of the solves the tick advanced
+    c.last_ms = ms / batch;
+    int64_t elems = 0;  // elements of the solves the ticks advanced
     for (auto* sv : c.slots)
         if (sv && sv->desc.start_tick <= done_tick) elems += sv->desc.E;
-    c.ticks_done += 1;
+    c.ticks_done += batch;
     c.busy_ms += ms;
-    c.dof_updates += (double)elems * c.np * c.ns * 5.0;
+    c.dof_updates += (double)elems * c.np * c.ns * 5.0 * batch;
     if (c.tune_done < 2 * c.ntiles) {
         // normalise by the elements of the tick so that ticks of different batches compare
         c.tune_ms[c.last_tile] += elems > 0 ? ms / (double)elems : ms;
@@ -548,13 +590,13 @@ cudaError_t finish_tick(rb200_server* s, Class& c) {
             c.tile = best;
         }
     }
-    c.tick += 1;
-    s->ticks += 1;
+    c.tick += batch;
+    s->ticks += batch;
     bool status_read = false;
     for (int i = 0; i < kMaxSolvesPerClass; ++i) {
         Solve* sv = c.slots[i];
-        if (!sv || sv->desc.start_tick > done_tick) continue;  // admitted while the tick ran
-        sv->steps_done += 1;
+        if (!sv || sv->desc.start_tick > done_tick) continue;  // admitted while the ticks ran
+        sv->steps_done += batch;
         Req& r = *sv->req;
         if (sv->steps_done < r.nsteps) continue;
         if (c.pipelined && !status_read) {  // a bounded wait of the pipelined kernel gave up: the result is void
@@ -628,6 +670,9 @@ void completion_loop(rb200_server* s) {
 // the step time of large ones.
 void server_loop(rb200_server* s) {
     cudaSetDevice(s->device);
+    // this thread's sleeps end within a microsecond of their time (the default slack of 50 us
+    // is more than a tick of a small class)
+    prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);
     std::unique_lock<std::mutex> lk(s->mu);
     while (true) {
         if (s->err_status != RB200_OK) break;
@@ -649,11 +694,11 @@ void server_loop(rb200_server* s) {
                     e = qe;
                     break;
                 }
-                e = finish_tick(s, c);
+                e = finish_ticks(s, c);
                 if (e != cudaSuccess) break;
             }
             if (c.active > 0) {
-                e = launch_tick(c);
+                e = launch_ticks(c);
                 if (e != cudaSuccess) break;
                 ++in_flight;
             }

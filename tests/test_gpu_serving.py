@@ -232,3 +232,21 @@ def test_small_poisson_stream(rb, S):
     assert st["completed"] == 40 and st["arena_used"] == 0
     assert all(np.all(np.isfinite(q)) for q in res["results"])
     assert res["solves_per_s"] > 0 and res["dof_updates_per_s"] > 0
+
+
+def test_ticks_enqueued_together(rb, S):
+    """One class of solves whose step counts end inside, at and beyond the ticks that are
+    enqueued at once, joining while others run, on chunk tables of one tile a chunk (9 elements)
+    to many (11^3 and two more): each equals its run alone, bit for bit."""
+    K = [(3, 3, 1), (11, 11, 11), (5, 4, 3), (8, 8, 8), (2, 2, 2)]
+    steps = [1, 40, 7, 16, 33]
+    specs = [_spec(S, 3, 4, 1, k, n, prec=1) for k, n in zip(K, steps)]
+    alone = []
+    for s in specs:
+        with S.Server(arena_bytes=1 << 28) as one:
+            alone.append(one.wait(one.submit(s))[0])
+    with S.Server(arena_bytes=1 << 28) as srv:
+        for _ in range(2):  # the second time past the autotuner's ticks
+            tickets = [srv.submit(s) for s in specs]
+            for t, ref in zip(tickets, alone):
+                assert np.array_equal(srv.wait(t)[0], ref)
