@@ -140,36 +140,6 @@ __device__ __forceinline__ int thread_index() {
     return t;
 }
 
-// Reciprocal and square root by Newton's iteration from the hardware's approximations (PTX
-// rcp.approx and rsqrt.approx: some 20 bits in FP64, 23 in FP32), good to about a rounding.
-// The compiler's own divide and root branch to a slow path for extreme arguments, which cuts
-// the unrolled pair loops into blocks that cannot overlap; these do not branch.  Arguments
-// are densities, pressures and their like: normal and far from the ends of the range.
-__device__ __forceinline__ double rcp(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
-}
-__device__ __forceinline__ float rcp(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
-}
-__device__ __forceinline__ double root(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
-    const double s = x * y;
-    return x == 0.0 ? x : fma(0.5 * y, fma(-s, s, x), s);
-}
-__device__ __forceinline__ float root(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float s = x * y;
-    return x == 0.0f ? x : fmaf(0.5f * y, fmaf(-s, s, x), s);
-}
-
 // gamma, gamma - 1 and 1 / (2 (gamma - 1)) (kernel parameters: no registers)
 template <typename T>
 __device__ __forceinline__ T gas(const PipeArgs& A, int i) {
@@ -327,7 +297,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 const int n = p0_node(h);
                 if (NP % NT != 0 && n >= NP) continue;
                 const T rho = (T)sm.q[buf][0][n];
-                const T rinv = line::rcp(rho);
+                const T rinv = rcp(rho);
                 const T m0 = (T)sm.q[buf][1][n], m1 = (T)sm.q[buf][2][n], m2 = (T)sm.q[buf][3][n];
                 const T u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
                 const T rhoe = (T)sm.q[buf][4][n];
@@ -345,7 +315,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                     o[1] = u0;
                     o[2] = u1;
                     o[3] = u2;
-                    o[4] = T(0.5) * rho * line::rcp(p);
+                    o[4] = T(0.5) * rho * rcp(p);
                     o[5] = u0 * u0 + u1 * u1 + u2 * u2;
                 } else {  // rho, u, E, p
                     o[0] = rho;
@@ -492,7 +462,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 auto two_point = [&](const T (&x)[NAUX], const T (&y)[NAUX], const T q, T (&F)[NS], auto exact) {
                     const T ua0 = (x[1] + y[1]) * T(0.5), ua1 = (x[2] + y[2]) * T(0.5), ua2 = (x[3] + y[3]) * T(0.5);
                     const T rs = x[0] + y[0], bs = x[4] + y[4];
-                    const T ir = line::rcp(rs), ib = line::rcp(bs);
+                    const T ir = rcp(rs), ib = rcp(bs);
                     T rlog, iblog;
                     if constexpr (decltype(exact)::value) {
                         rlog = log_mean(x[0], y[0], ir);
@@ -577,7 +547,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                     Em = rm * (T(2) * o[0][4]);
                 } else if constexpr (COMBO == EUL_EC) {
                     rm = o[0][0];
-                    pm = rm * (T(0.5) * line::rcp(o[0][4]));
+                    pm = rm * (T(0.5) * rcp(o[0][4]));
                     Em = pm * (T(2) * line::gas<T>(A, 2)) + T(0.5) * rm * o[0][5];
                 } else {
                     rm = o[0][0];
@@ -586,7 +556,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 }
 #pragma unroll
                 for (int d = 0; d < 3; ++d) um[d] = COMBO == EUL_KG ? T(2) * o[0][1 + d] : o[0][1 + d];
-                const T rp = (T)tr[DIR][0], Ep = (T)tr[DIR][4], rinv = line::rcp(rp);
+                const T rp = (T)tr[DIR][0], Ep = (T)tr[DIR][4], rinv = rcp(rp);
                 T mp[3], up[3];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
@@ -596,7 +566,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 const T pp = line::gas<T>(A, 1) * (Ep - (mp[0] * mp[0] + mp[1] * mp[1] + mp[2] * mp[2]) * (T(0.5) * rinv));
                 const T unm = um[DIR] * sn, unp = up[DIR] * sn, mnm = rm * unm, mnp = mp[DIR] * sn;
                 // the larger wave speed |u.n| + sqrt(gamma p / rho) (euler.jl:62-68)
-                const T wm = fabs(unm) + line::root(line::gas<T>(A, 0) * pm * line::rcp(rm)), wp = fabs(unp) + line::root(line::gas<T>(A, 0) * pp * rinv);
+                const T wm = fabs(unm) + root(line::gas<T>(A, 0) * pm * rcp(rm)), wp = fabs(unp) + root(line::gas<T>(A, 0) * pp * rinv);
                 const T mx = A.surface_rusanov ? fmax(wm, wp) : T(0);
                 // normal fluxes of both sides (euler.jl:50-60 with n = sn e_dir), field by field
 #pragma unroll

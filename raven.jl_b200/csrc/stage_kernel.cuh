@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "rb200_internal.h"
 #include "surface_fluxes.cuh"
 
@@ -387,101 +389,125 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
     for (int s = 0; s < NS; ++s) acc[s] = T(0);
     const int dmask = A.dir_mask ? A.dir_mask : 7;  // DGSEM(; directions)
+    constexpr bool kSharedD = sizeof(T) == 4 || DIM < 3;
     [[maybe_unused]] const T ec_inv_2gm1 = T(1) / (T(2) * (T)(A.gamma - 1.0));
 
+    // EC: the pairs' logarithmic means by their power series, without branches; a node one of whose
+    // pairs lies beyond it takes its sums again with the logarithms
+    [[maybe_unused]] bool far = false;
+    auto volume = [&](auto exact) {
+        constexpr int kUnroll = decltype(exact)::value ? 1 : NQ;
 #pragma unroll
-    for (int dir = 0; dir < DIM; ++dir) {
-        if (!((dmask >> dir) & 1)) continue;
-        const int stride = dir == 0 ? 1 : (dir == 1 ? NQ : NQ * NQ);
-        const int idd = id[dir];
-        const int base = n - idd * stride;
+        for (int dir = 0; dir < DIM; ++dir) {
+            if (!((dmask >> dir) & 1)) continue;
+            const int stride = dir == 0 ? 1 : (dir == 1 ? NQ : NQ * NQ);
+            const int idd = id[dir];
+            const int base = n - idd * stride;
+#pragma unroll kUnroll
+            for (int a = 0; a < NQ; ++a) {
+                const int na = base + a * stride;
+                // D[a, id]: from shared memory, but 3-D FP64 from the parameters (each measured faster)
+                const T Dai = kSharedD ? sD[a + NQ * idd] : (T)A.D[a + NQ * idd];
+                if constexpr (COMBO == ADV_WEAK) {
+                    acc[0] += Dai * aux[dir * NP + na];
+                } else if constexpr (COMBO == EUL_WEAK) {
 #pragma unroll
-        for (int a = 0; a < NQ; ++a) {
-            const int na = base + a * stride;
-            // D[a, id]: FP32 from shared memory (measured faster), FP64 from the parameters
-            const T Dai = sizeof(T) == 4 ? sD[a + NQ * idd] : (T)A.D[a + NQ * idd];
-            if constexpr (COMBO == ADV_WEAK) {
-                acc[0] += Dai * aux[dir * NP + na];
-            } else if constexpr (COMBO == EUL_WEAK) {
-#pragma unroll
-                for (int s = 0; s < NS; ++s) acc[s] += Dai * aux[(dir * NS + s) * NP + na];
-            } else {
-                const T Dia = sizeof(T) == 4 ? sD[idd + NQ * a] : (T)A.D[idd + NQ * a];  // D[id, a]
-                // metric combination G_d = D[a,id] l_g[a][d] - D[id,a] l_g[i][d]
-                T G[DIM];
-                if constexpr (AFF) {
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) G[d] = T(0);
-                    G[dir] = sub_rn(mul_rn(Dai, lgs[dir * NP + na]), mul_rn(Dia, lg[dir]));
+                    for (int s = 0; s < NS; ++s) acc[s] += Dai * aux[(dir * NS + s) * NP + na];
                 } else {
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d)
-                        G[d] = sub_rn(mul_rn(Dai, lgs[(dir * DIM + d) * NP + na]), mul_rn(Dia, lg[dir * DIM + d]));
-                }
-                if constexpr (COMBO == ADV_FDC) {
-                    T aG = (T)A.adv[0] * G[0];
-#pragma unroll
-                    for (int d = 1; d < DIM; ++d) aG += (T)A.adv[d] * G[d];
-                    acc[0] += (own[0] + aux[na]) * aG;
-                } else if constexpr (COMBO == EUL_FDC) {
-#pragma unroll
-                    for (int s = 0; s < NS; ++s) {
-                        T v = T(0);
-#pragma unroll
-                        for (int d = 0; d < DIM; ++d) v += (own[d * NS + s] + aux[(d * NS + s) * NP + na]) * G[d];
-                        acc[s] += v;
-                    }
-                } else if constexpr (COMBO == EUL_KG) {
-                    const T rb = own[0] + aux[na];
-                    T ub[DIM];
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) ub[d] = own[1 + d] + aux[(1 + d) * NP + na];
-                    const T eb = own[DIM + 1] + aux[(DIM + 1) * NP + na];
-                    const T pb = own[DIM + 2] + aux[(DIM + 2) * NP + na];
-                    T un;
+                    const T Dia = kSharedD ? sD[idd + NQ * a] : (T)A.D[idd + NQ * a];  // D[id, a]
+                    // metric combination G_d = D[a,id] l_g[a][d] - D[id,a] l_g[i][d]
+                    T G[DIM];
                     if constexpr (AFF) {
-                        un = ub[dir] * G[dir];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) G[d] = T(0);
+                        G[dir] = sub_rn(mul_rn(Dai, lgs[dir * NP + na]), mul_rn(Dia, lg[dir]));
                     } else {
-                        un = ub[0] * G[0];
 #pragma unroll
-                        for (int d = 1; d < DIM; ++d) un += ub[d] * G[d];
+                        for (int d = 0; d < DIM; ++d)
+                            G[d] = sub_rn(mul_rn(Dai, lgs[(dir * DIM + d) * NP + na]), mul_rn(Dia, lg[dir * DIM + d]));
                     }
-                    const T f1 = rb * un;
-                    acc[0] += f1;
+                    if constexpr (COMBO == ADV_FDC) {
+                        T aG = (T)A.adv[0] * G[0];
 #pragma unroll
-                    for (int b = 0; b < DIM; ++b) {
-                        if (AFF && b != dir) acc[1 + b] += f1 * ub[b];
-                        else acc[1 + b] += f1 * ub[b] + pb * G[b];
+                        for (int d = 1; d < DIM; ++d) aG += (T)A.adv[d] * G[d];
+                        acc[0] += (own[0] + aux[na]) * aG;
+                    } else if constexpr (COMBO == EUL_FDC) {
+#pragma unroll
+                        for (int s = 0; s < NS; ++s) {
+                            T v = T(0);
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) v += (own[d * NS + s] + aux[(d * NS + s) * NP + na]) * G[d];
+                            acc[s] += v;
+                        }
+                    } else if constexpr (COMBO == EUL_KG) {
+                        const T rb = own[0] + aux[na];
+                        T ub[DIM];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) ub[d] = own[1 + d] + aux[(1 + d) * NP + na];
+                        const T eb = own[DIM + 1] + aux[(DIM + 1) * NP + na];
+                        const T pb = own[DIM + 2] + aux[(DIM + 2) * NP + na];
+                        T un;
+                        if constexpr (AFF) {
+                            un = ub[dir] * G[dir];
+                        } else {
+                            un = ub[0] * G[0];
+#pragma unroll
+                            for (int d = 1; d < DIM; ++d) un += ub[d] * G[d];
+                        }
+                        const T f1 = rb * un;
+                        acc[0] += f1;
+#pragma unroll
+                        for (int b = 0; b < DIM; ++b) {
+                            if (AFF && b != dir) acc[1 + b] += f1 * ub[b];
+                            else acc[1 + b] += f1 * ub[b] + pb * G[b];
+                        }
+                        acc[DIM + 1] += un * (rb * eb + pb);
+                    } else {  // EUL_EC
+                        const T r2 = aux[na];
+                        T u2[DIM], ua[DIM];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) {
+                            u2[d] = aux[(1 + d) * NP + na];
+                            ua[d] = (own[1 + d] + u2[d]) * T(0.5);
+                        }
+                        const T b2 = aux[(DIM + 1) * NP + na];
+                        const T uu2 = aux[(DIM + 2) * NP + na];
+                        const T u2a = (own[DIM + 2] + uu2) * T(0.5);
+                        const T ir = rcp(own[0] + r2), ib = rcp(own[DIM + 1] + b2);
+                        T rlog, iblog;
+                        if constexpr (decltype(exact)::value) {
+                            rlog = log_mean(own[0], r2, ir);
+                            iblog = inverse_log_mean(own[DIM + 1], b2, ib);
+                        } else {
+                            const T fr = (own[0] - r2) * ir, fb = (own[DIM + 1] - b2) * ib, ur = fr * fr, ub = fb * fb;
+                            rlog = (T(0.5) * (own[0] + r2)) * log_mean_inverse_series(ur);
+                            iblog = (T(2) * ib) * log_mean_series(ub);
+                            far |= !(ur < T(0.01)) | !(ub < T(0.01));
+                        }
+                        const T pt = (T(0.5) * (own[0] + r2)) * ib;  // rho_avg / (2 b_avg)
+                        const T c = ec_inv_2gm1 * iblog - u2a * T(0.5);
+                        T un = ua[0] * G[0], uaa = ua[0] * ua[0];
+#pragma unroll
+                        for (int d = 1; d < DIM; ++d) {
+                            un += ua[d] * G[d];
+                            uaa += ua[d] * ua[d];
+                        }
+                        const T f0 = rlog * un;
+                        acc[0] += f0;
+#pragma unroll
+                        for (int b = 0; b < DIM; ++b) acc[1 + b] += f0 * ua[b] + pt * G[b];
+                        acc[DIM + 1] += un * (c * rlog + rlog * uaa + pt);
                     }
-                    acc[DIM + 1] += un * (rb * eb + pb);
-                } else {  // EUL_EC
-                    const T r2 = aux[na];
-                    T u2[DIM], ua[DIM];
-#pragma unroll
-                    for (int d = 0; d < DIM; ++d) {
-                        u2[d] = aux[(1 + d) * NP + na];
-                        ua[d] = (own[1 + d] + u2[d]) * T(0.5);
-                    }
-                    const T b2 = aux[(DIM + 1) * NP + na];
-                    const T uu2 = aux[(DIM + 2) * NP + na];
-                    const T u2a = (own[DIM + 2] + uu2) * T(0.5);
-                    const T ir = T(1) / (own[0] + r2), ib = T(1) / (own[DIM + 1] + b2);
-                    const T rlog = log_mean(own[0], r2, ir);
-                    const T pt = (T(0.5) * (own[0] + r2)) * ib;  // rho_avg / (2 b_avg)
-                    const T c = ec_inv_2gm1 * inverse_log_mean(own[DIM + 1], b2, ib) - u2a * T(0.5);
-                    T un = ua[0] * G[0], uaa = ua[0] * ua[0];
-#pragma unroll
-                    for (int d = 1; d < DIM; ++d) {
-                        un += ua[d] * G[d];
-                        uaa += ua[d] * ua[d];
-                    }
-                    const T f0 = rlog * un;
-                    acc[0] += f0;
-#pragma unroll
-                    for (int b = 0; b < DIM; ++b) acc[1 + b] += f0 * ua[b] + pt * G[b];
-                    acc[DIM + 1] += un * (c * rlog + rlog * uaa + pt);
                 }
             }
+        }
+    };
+    volume(std::false_type{});
+    if constexpr (COMBO == EUL_EC) {
+        if (far) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) acc[s] = T(0);
+            volume(std::true_type{});
         }
     }
 

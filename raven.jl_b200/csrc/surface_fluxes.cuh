@@ -12,6 +12,36 @@
 
 namespace rb200 {
 
+// Reciprocal and square root by Newton's iteration from the hardware's approximations (PTX
+// rcp.approx and rsqrt.approx: some 20 bits in FP64, 23 in FP32), good to about a rounding.
+// The compiler's own divide and root branch to a slow path for extreme arguments, which cuts
+// the unrolled pair loops into blocks that cannot overlap; these do not branch.  Arguments
+// are densities, pressures and their like: normal and far from the ends of the range.
+__device__ __forceinline__ double rcp(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+__device__ __forceinline__ double root(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+    const double s = x * y;
+    return x == 0.0 ? x : fma(0.5 * y, fma(-s, s, x), s);
+}
+__device__ __forceinline__ float root(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = x * y;
+    return x == 0.0f ? x : fmaf(0.5f * y, fmaf(-s, s, x), s);
+}
+
 // The logarithmic mean (a - b) / log(a / b) of logavg (numericalfluxes.jl:9-22) and its
 // reciprocal.  With f = (a - b) / (a + b), u = f^2 and F(u) = atanh(f) / f = sum u^k / (2k + 1),
 // the mean is (a + b) / (2 F) (Ismail and Roe 2009).  Below |f| = 0.1 (a ratio of 1.22: the
