@@ -224,8 +224,7 @@ cudaError_t launch_any(rb200_handle* h, const StageArgs& a, cudaStream_t st) {
         std::memset(&c, 0, sizeof(c));
         c.q_in = a.q_in;
         c.q_out = a.q_out;
-        if (h->prec == RB200_PRECISION_FP64) c.dq64 = static_cast<double*>(a.dq);
-        else c.dq = static_cast<float*>(a.dq);
+        c.dq = a.dq;
         c.vgeo = h->d_vgeo;
         c.sgeo = h->d_sgeo;
         c.nbr = h->d_nbr;
@@ -236,11 +235,12 @@ cudaError_t launch_any(rb200_handle* h, const StageArgs& a, cudaStream_t st) {
         c.surface_rusanov = a.surface_rusanov;
         c.rka = a.rka;
         c.rkb_dt = a.rkb_dt;
-        c.gamma = a.gamma;
+        c.gas[0] = a.gamma, c.gas[1] = a.gamma - 1.0;
+        for (int i = 0; i < 2; ++i) c.gasf[i] = (float)c.gas[i];
         std::memcpy(c.D, h->D, sizeof(c.D));
+        for (int i = 0; i < 64; ++i) c.Df[i] = (float)h->D[i];
         const int grid = (int)std::min<int64_t>(h->pipe_curved_grid, a.E - a.e_begin);
-        return h->prec == RB200_PRECISION_FP64 ? launch_pipelined_curved64(c, grid, st)
-                                               : launch_pipelined_curved(c, grid, st);
+        return launch_pipelined_curved(h->prec, c, grid, st);
     }
     const bool eligible = all_dirs && h->kernel_path == 0 && h->pipe_grid > 0 && aligned16(a.q_in) && aligned16(a.dq) &&
                           (!stage_mode || aligned16(a.q_out)) &&
@@ -773,13 +773,12 @@ rb200_status rb200_create(const rb200_desc* d, rb200_handle** out) {
         cudaGetLastError();
     }
     if (dim == 3 && nq == 8 && !affine && !general && h->combo == EUL_KG && !entropy_flux && h->d_vgeo && h->d_sgeo &&
-        aligned16(h->d_vgeo) && aligned16(h->d_sgeo)) {
-        // curved 3-D Nq = 8 Kennedy-Gruber: the curved pipelined kernel of the handle's precision
+        aligned16(h->d_vgeo) && ((uintptr_t)h->d_sgeo & 31u) == 0 && pipe_odd_derivative(nq, h->D)) {
+        // curved 3-D Nq = 8 Kennedy-Gruber: the curved pipelined kernel
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const int per_sm = h->prec == RB200_PRECISION_FP64 ? pipelined_curved64_blocks_per_sm()
-                                                           : pipelined_curved_blocks_per_sm();
+        const int per_sm = pipelined_curved_blocks_per_sm(h->prec);
         h->pipe_curved_grid = per_sm > 0 ? per_sm * nsm : 0;
         cudaGetLastError();
     }

@@ -124,7 +124,21 @@ constexpr int min_ctas() {
     return m[Q - 4][sizeof(T) == 4];
 }
 
-// Stores 4 consecutive values, 32 bytes at once where the address allows it (`wide`)
+// 4 consecutive values, 32 bytes at once where the address allows it (`wide`).  The load is not
+// volatile, so that the compiler may place it where registers allow: where it must stay behind
+// a wait of the kernel, `p` comes from after().
+__device__ __forceinline__ size_t after(size_t x) {
+    asm volatile("mov.u64 %0, %0;" : "+l"(x)::"memory");
+    return x;
+}
+__device__ __forceinline__ void load4(const double* p, bool wide, double (&v)[4]) {
+    if (wide) {
+        asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+    } else {
+        const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+        v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+    }
+}
 __device__ __forceinline__ void store4(double* p, bool wide, const double (&v)[4]) {
     if (wide) {
         asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");

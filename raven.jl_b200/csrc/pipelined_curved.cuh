@@ -1,46 +1,38 @@
-// Persistent, bulk-copy-pipelined LSRK stage kernel for 3-D hexahedra with Nq = 8 on
-// curved (warped) grids: Kennedy-Gruber flux differencing, FP32 bulk arithmetic, FP64
-// state, metrics and LSRK state update.
+// Persistent LSRK stage kernel of the Euler law on curved 3-D grids with Nq = 8, Kennedy-Gruber
+// flux differencing, FP64 or FP32 bulk (stage modes).
 //
-// The curved form of esvolumeterm_dir! (src/balancelaws/dgsem.jl:514-608) contracts the
-// two-point flux of nodes i and a on a line in direction dir with
-//     G_d = D[a,i] l_g[a][dir][d] - D[i,a] l_g[i][dir][d],   l_g = wJ dRdX (vgeo rows),
-// and the result is scaled by MJI.  The surface term (dgsem.jl:733-784) takes the
-// Rusanov or central flux with the face normal n and subtracts (wsJ nf) MJI.
+// The half-line design of line_kernel.cuh: 128 threads share an element, in each direction a
+// thread owns the four nodes from one end of a line to its middle, takes the pairs among them
+// once for both nodes, meets the other half's nodes one by one, and adds the face flux of its
+// first node, which is the line's end.  z, then y, then x lines; sums pass between the
+// directions through shared memory.  What a curved grid adds:
+// * a pair's flux is contracted with G = D[a,i] l_g[a] - D[i,a] l_g[i] (esvolumeterm_dir!,
+//   src/balancelaws/dgsem.jl:576-600; l_g = wJ dRdX[dir,:], the rows of vgeo), which is skew in
+//   (a, i), and odd under reflection of the line like D;
+// * each direction needs only its own three rows, so the rows arrive by one bulk copy a
+//   direction (12 KB), into buffers that are free again when their direction is done: z's one
+//   element ahead, y's and x's (with MJI) while z's pairs run.  They stay FP64 in shared memory,
+//   FP32 bulk converts them as it reads;
+// * the face normal and wsJ are loaded with the neighbour's trace, 32 bytes a thread.
 //
-// Each CTA owns a strided set of elements; two CTAs share an SM.  Per element:
-// * the state q and the face geometry (n, wsJ for the 384 face nodes) arrive by 1-D
-//   bulk copies (cp.async.bulk, completion on mbarriers): q is issued one element ahead,
-//   right after the partner values of the current element are built from it; the face
-//   geometry after the current element's faces are done;
-// * the FP32 LSRK register arrives by a bulk copy issued at the start of the element;
-// * each thread loads the metric rows and MJI of its two nodes from global memory before
-//   it waits for q, so that the loads overlap that wait;
-// * the neighbour face traces arrive with cp.async during the volume term;
-// * the element's own old q is read at the end (L2-resident: it arrived by bulk copy).
+// What bounds it: HBM (256 B/node in FP64, 220 in FP32 bulk: 6.0 and 5.1 K cycles an element and
+// SM at the measured peak) and, in FP64, the FP64 pipe (4.5 K).  The kernels before this one (256
+// threads, each node its full lines of partners with their metric rows) took 16.5 and 12.2 K, and
+// this one 12.4 and 8.5 K: B200, one LSRK(5,4) step, FP64 13^3 634 -> 477 us, FP32 bulk 16^3 879 ->
+// 610.  Two CTAs of 128 threads share an SM (255 registers a thread in FP64; shared memory 107
+// and 83 KB a CTA): 8 warps do not cover the latencies between the two barriers.
 //
-// A thread owns nodes t and t + 256 (same i, j; k and k + 4), so their z partners are
-// loaded once.  Every wait on an mbarrier is bounded: after kWaitLimit polls the CTA
-// records RB200 status TIMEOUT in *A.status and returns.
+// Every mbarrier wait is bounded: on expiry the CTA records RB200 status TIMEOUT and returns.
 #pragma once
 
-#include "pipelined_kernel.cuh"
-
-// unroll factor of the curved kernels' pair loops over partners (8, full: measured 3.8 % (FP32
-// bulk) and 2.6 % (FP64) faster than 2 on the warped 32^3 grid, 128 registers, no spills)
-#ifndef RB200_CURVED_UNROLL
-#define RB200_CURVED_UNROLL 8
-#endif
+#include "line_kernel.cuh"
 
 namespace rb200 {
-
-constexpr int kCurvedUnroll = RB200_CURVED_UNROLL;
 
 struct PipeCurvedArgs {
     const double* q_in;
     double* q_out;
-    float* dq;               // FP32 LSRK register (FP32-bulk kernel)
-    double* dq64;            // FP64 LSRK register (FP64 kernel)
+    void* dq;                // LSRK register, float* in FP32 bulk
     const double* vgeo;      // (512, 11, E): wJ dRdX[dir][d] (dir-major), MJI, MJ
     const double* sgeo;      // (4, 384, E): n, wsJ per face node
     const int32_t* nbr;      // (6, E)
@@ -49,299 +41,353 @@ struct PipeCurvedArgs {
     int64_t e_begin;
     int32_t mode;            // MODE_STAGE or MODE_STAGE_FIRST
     int32_t surface_rusanov;
-    double rka, rkb_dt, gamma;
-    double D[64];            // D[i + 8 j] = l_j'(r_i)
+    double rka, rkb_dt;
+    double gas[3];           // gamma, gamma - 1
+    float gasf[3];
+    double D[64];            // D[i + 8 j] = l_j'(r_i), odd under reflection of the line
+    float Df[64];
 };
 
 namespace pipec {
 
-using pipe::NAUX;
-using pipe::NP;
-using pipe::NPP;
-using pipe::NQ;
-using pipe::NS;
-using pipe::NSLOT;
-using pipe::PAD;
-constexpr int NT = 256, NVG = 11;
+constexpr int Q = 8, NP = 512, NFP = 64, NT = 128;
+using LS = line::Shape<Q>;
 
+template <typename T>
 struct Smem {
-    double q[NS][NP];                 // element state (bulk copy)
-    double sg[NSLOT][4];              // face normal and wsJ per face slot (bulk copy)
-    __align__(16) float dqb[NS][NP];  // the element's LSRK register (bulk copy)
-    float4 auxa[NPP];                 // partner values: rho/2, u/2
-    float2 auxb[NPP];                 // e/2, p/2
-    float4 lgd[3][NPP];               // l_g[dir][0..2] of each node
-    double slot[NS][NSLOT];           // neighbour trace, then (wsJ nf) MJI per face slot
-    float mji[NP];
-    float D[NQ][NQ];                  // D[i][j] = l_j'(r_i)
-    int32_t nb[2][8];                 // neighbours of the current / next element
-    uint64_t barq, bars, bard;        // arrivals of q, face geometry, register
+    __align__(16) double q[pipe::NS][NP];   // state of the element, then (after #1) of the next one
+    __align__(16) double geo[10][NP];       // rows l_g[dir][d] of the element, and MJI
+    pipe::Partners<T, NP + LS::PAD16, NP + LS::PAD8> aux;
+    __align__(16) T acc[pipe::NS][NP];      // sums of the directions done
+    int32_t nb[2][8];                       // neighbours of the current / next element
+    uint64_t bar_q, bar_geo[3];
 };
+
+// D[i, j] as a kernel parameter in type T
+template <typename T>
+__device__ __forceinline__ T dpar(const PipeCurvedArgs& A, int i, int j) {
+    if constexpr (sizeof(T) == 8) return A.D[i + 8 * j];
+    else return A.Df[i + 8 * j];
+}
+template <typename T>
+__device__ __forceinline__ T gas(const PipeCurvedArgs& A, int i) {
+    if constexpr (sizeof(T) == 8) return A.gas[i];
+    else return A.gasf[i];
+}
 
 }  // namespace pipec
 
-template <int COMBO>
-__global__ void __launch_bounds__(256, 2) pipelined_curved_kernel(const __grid_constant__ PipeCurvedArgs A) {
+template <typename T>
+__global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __grid_constant__ PipeCurvedArgs A) {
     using namespace pipe;
-    using namespace pipec;
-    static_assert(COMBO == EUL_KG, "the curved pipelined kernel implements Kennedy-Gruber");
+    using pipec::LS;
+    constexpr int Q = pipec::Q, NP = pipec::NP, NFP = pipec::NFP, H0 = 4;
     extern __shared__ __align__(128) unsigned char pipe_smem_raw[];
-    pipec::Smem& sm = *reinterpret_cast<pipec::Smem*>(pipe_smem_raw);
+    pipec::Smem<T>& sm = *reinterpret_cast<pipec::Smem<T>*>(pipe_smem_raw);
     const int t = threadIdx.x;
-    const int ii = t & 7, jj = (t >> 3) & 7, k0 = t >> 6;
-    const bool read_dq = A.mode == MODE_STAGE;
-    const uint32_t qbytes = NS * NP * sizeof(double), sgbytes = NSLOT * 4 * sizeof(double),
-                   dqbytes = NS * NP * sizeof(float);
-    const float gm1 = (float)(A.gamma - 1.0), gam = (float)A.gamma;
+    const bool reads_dq = A.mode == MODE_STAGE;
+    const int E = (int)A.E;
+    // the rows of direction dir (x: with MJI) of element e into their place
+    auto fetch_rows = [&](int dir, int64_t e) {
+        const double* src = A.vgeo + (size_t)e * 11 * NP;
+        constexpr uint32_t bytes = 3 * NP * sizeof(double);
+        mbar_expect_tx(&sm.bar_geo[dir], bytes + (dir == 0 ? NP * sizeof(double) : 0));
+        bulk_g2s(&sm.geo[3 * dir][0], src + 3 * dir * NP, bytes, &sm.bar_geo[dir]);
+        if (dir == 0) bulk_g2s(&sm.geo[9][0], src + 9 * NP, NP * sizeof(double), &sm.bar_geo[0]);
+    };
+    auto fetch_state = [&](int64_t e) {
+        mbar_expect_tx(&sm.bar_q, NS * NP * sizeof(double));
+        bulk_g2s(&sm.q[0][0], A.q_in + (size_t)e * NS * NP, NS * NP * sizeof(double), &sm.bar_q);
+    };
 
+    int e = (int)A.e_begin + blockIdx.x;
     if (t == 0) {
-        mbar_init(&sm.barq, 1);
-        mbar_init(&sm.bars, 1);
-        mbar_init(&sm.bard, 1);
+        mbar_init(&sm.bar_q, 1);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) mbar_init(&sm.bar_geo[d], 1);
         fence_mbar_init();
+        if (e < E) {
+            fetch_rows(2, e);  // geometry: written by no kernel
+            fetch_state(e);
+        }
     }
-    for (int c = t; c < 64; c += NT) sm.D[c & 7][c >> 3] = (float)A.D[c];
-    int64_t e = A.e_begin + blockIdx.x;
-    if (t < 6 && e < A.E) cp_async4(&sm.nb[0][t], A.nbr + 6 * e + t);
+    if (t < 6 && e < E) cp_async4(&sm.nb[0][t], A.nbr + (size_t)6 * e + t);
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    if (t == 0 && e < A.E) {
-        mbar_expect_tx(&sm.barq, qbytes);
-        bulk_g2s(&sm.q[0][0], A.q_in + (size_t)e * NS * NP, qbytes, &sm.barq);
-        mbar_expect_tx(&sm.bars, sgbytes);
-        bulk_g2s(&sm.sg[0][0], A.sgeo + (size_t)e * NSLOT * 4, sgbytes, &sm.bars);
-    }
-    uint32_t phq = 0, phs = 0, phd = 0;
-    for (int buf = 0; e < A.E; buf ^= 1, e += gridDim.x) {
-        const int64_t en = e + gridDim.x;  // the next element of this CTA
-        // ---- metric rows and MJI of the thread's nodes (overlap the wait for q)
-        double vgl[2][9], mjid[2];
-        {
-            const double* vg = A.vgeo + (size_t)e * NVG * NP + t;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                for (int c = 0; c < 9; ++c) vgl[h][c] = __ldg(vg + c * NP + NT * h);
-                mjid[h] = __ldg(vg + 9 * NP + NT * h);
-            }
-        }
-        if (__syncthreads_or(!bounded_wait(&sm.barq, phq))) {
-            if (t == 0) atomicExch(A.status, kStatusTimeout);
-            return;
-        }
-        phq ^= 1;
-        // ---- partner values, metric rows and MJI into shared memory
-        float own[2][NAUX], lgo[2][9], mjiT[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int n = t + NT * h;
-            const float rho = (float)sm.q[0][n];
-            const float rinv = 1.f / rho;
-            const float m0 = (float)sm.q[1][n], m1 = (float)sm.q[2][n], m2 = (float)sm.q[3][n];
-            const float rhoe = (float)sm.q[4][n];
-            const float u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
-            const float p = gm1 * (rhoe - (m0 * m0 + m1 * m1 + m2 * m2) / (2.f * rho));
-            own[h][0] = rho * 0.5f;
-            own[h][1] = u0 * 0.5f;
-            own[h][2] = u1 * 0.5f;
-            own[h][3] = u2 * 0.5f;
-            own[h][4] = (rhoe / rho) * 0.5f;
-            own[h][5] = p * 0.5f;
-            sm.auxa[PAD(n)] = make_float4(own[h][0], own[h][1], own[h][2], own[h][3]);
-            sm.auxb[PAD(n)] = make_float2(own[h][4], own[h][5]);
-#pragma unroll
-            for (int c = 0; c < 9; ++c) lgo[h][c] = (float)vgl[h][c];
-#pragma unroll
-            for (int dir = 0; dir < 3; ++dir)
-                sm.lgd[dir][PAD(n)] = make_float4(lgo[h][3 * dir], lgo[h][3 * dir + 1], lgo[h][3 * dir + 2], 0.f);
-            mjiT[h] = (float)mjid[h];
-            sm.mji[n] = mjiT[h];
-        }
-        __syncthreads();  // #1: partner values ready; q is free
-        if (t == 0) {
-            fence_proxy_async();  // q and dqb were last read by the generic proxy
-            if (en < A.E) {  // the next element's state
-                mbar_expect_tx(&sm.barq, qbytes);
-                bulk_g2s(&sm.q[0][0], A.q_in + (size_t)en * NS * NP, qbytes, &sm.barq);
-            }
-            if (read_dq) {  // this element's register (the previous element's final phase is done)
-                mbar_expect_tx(&sm.bard, dqbytes);
-                bulk_g2s(&sm.dqb[0][0], A.dq + (size_t)e * NS * NP, dqbytes, &sm.bard);
-            }
-        }
-        if (t < 6 && en < A.E) cp_async4(&sm.nb[buf ^ 1][t], A.nbr + 6 * en + t);
-        // neighbour traces of this thread's face slots t and t + 256
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const int slot = t + NT * sl;
-            if (slot >= NSLOT) continue;
-            int vn, opp;
-            slot_nodes(slot, vn, opp);
-            const int ne = sm.nb[buf][slot >> 6];
-            if (ne >= 0) {
-                const double* qn = A.q_in + (size_t)ne * NS * NP + opp;
-#pragma unroll
-                for (int s = 0; s < NS; ++s) cp_async8(&sm.slot[s][slot], qn + s * NP);
-            }
-        }
-        cp_async_commit();
 
-        // ---- volume term: pairs along x, y, z with the averaged metric combination G
-        float acc[2][NS];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int s = 0; s < NS; ++s) acc[h][s] = 0.f;
-        auto pair = [&](float (&ac)[NS], const float (&o)[NAUX], const float4 pa, const float2 pb, const float4 lp,
-                        const float* lo, const float Dai, const float Dia) {
-            float G[3];
-            // the self pair, whose G must cancel exactly, is never formed (a != i)
-            G[0] = fmaf(Dai, lp.x, -(Dia * lo[0]));
-            G[1] = fmaf(Dai, lp.y, -(Dia * lo[1]));
-            G[2] = fmaf(Dai, lp.z, -(Dia * lo[2]));
-            const float rb = o[0] + pa.x;
-            const float ub0 = o[1] + pa.y, ub1 = o[2] + pa.z, ub2 = o[3] + pa.w;
-            const float eb = o[4] + pb.x, pbar = o[5] + pb.y;
-            const float un = ub0 * G[0] + ub1 * G[1] + ub2 * G[2];
-            const float f1 = rb * un;
-            ac[0] += f1;
-            ac[1] += f1 * ub0 + pbar * G[0];
-            ac[2] += f1 * ub1 + pbar * G[1];
-            ac[3] += f1 * ub2 + pbar * G[2];
-            ac[4] += un * (rb * eb + pbar);
-        };
-#pragma unroll kCurvedUnroll
-        for (int a = 0; a < NQ; ++a) {
-            const float Dax = sm.D[a][ii], Dxa = sm.D[ii][a];
-            const float Day = sm.D[a][jj], Dya = sm.D[jj][a];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int kk = k0 + 4 * h;
-                if (a != ii) {
-                    const int na = a + 8 * (jj + 8 * kk);
-                    pair(acc[h], own[h], sm.auxa[PAD(na)], sm.auxb[PAD(na)], sm.lgd[0][PAD(na)], &lgo[h][0], Dax, Dxa);
-                }
-                if (a != jj) {
-                    const int na = ii + 8 * (a + 8 * kk);
-                    pair(acc[h], own[h], sm.auxa[PAD(na)], sm.auxb[PAD(na)], sm.lgd[1][PAD(na)], &lgo[h][3], Day, Dya);
-                }
-            }
-            const int nz = ii + 8 * (jj + 8 * a);
-            const float4 za = sm.auxa[PAD(nz)], zl = sm.lgd[2][PAD(nz)];
-            const float2 zb = sm.auxb[PAD(nz)];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int kk = k0 + 4 * h;
-                if (a != kk) pair(acc[h], own[h], za, zb, zl, &lgo[h][6], sm.D[a][kk], sm.D[kk][a]);
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int s = 0; s < NS; ++s) acc[h][s] = acc[h][s] * mjiT[h];
-
-        // ---- face-slot contributions (wsJ nf) MJI, written over the slot's trace
+    uint32_t ph = 0;     // parity of every copy: one of each an element
+    bool late = false;   // a wait of this thread ran out
+    for (int buf = 0; e < E; buf ^= 1, e += gridDim.x, ph ^= 1) {
+        const int en = e + (int)gridDim.x;
+        late |= !bounded_wait(&sm.bar_q, ph);
         cp_async_wait_all();
-        if (__syncthreads_or(!bounded_wait(&sm.bars, phs))) {  // also: the traces of every thread
-            if (t == 0) atomicExch(A.status, kStatusTimeout);
+        __syncwarp();  // the x phase of the previous element has read its planes' partner values
+        // ---- per-node partner values of the warp's two z planes: halves of rho, u, e, p
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const int n = (t & 31) + 32 * h + 128 * (t >> 5);
+            const T rho = (T)sm.q[0][n], rinv = rcp(rho);
+            const T m0 = (T)sm.q[1][n], m1 = (T)sm.q[2][n], m2 = (T)sm.q[3][n], rhoe = (T)sm.q[4][n];
+            const T u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
+            const T p = pipec::gas<T>(A, 1) * (rhoe - (m0 * m0 + m1 * m1 + m2 * m2) * (T(0.5) * rinv));
+            const T o[NAUX] = {rho * T(0.5), u0 * T(0.5), u1 * T(0.5), u2 * T(0.5), rhoe * rinv * T(0.5), p * T(0.5)};
+            sm.aux.put(LS::slot16(n), LS::slot8(n), o);
+        }
+        if (__syncthreads_or(late)) {  // #1: partner values ready; the state's and the rows' buffers are free
+            if (t == 0) {
+                atomicExch(A.status, kStatusTimeout);
+                bounded_wait(&sm.bar_geo[2], ph);
+            }
             return;
         }
-        phs ^= 1;
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const int slot = t + NT * sl;
-            if (slot >= NSLOT) continue;
-            const int f = slot >> 6;
-            int vn, opp;
-            slot_nodes(slot, vn, opp);
-            const bool open_face = sm.nb[buf][f] >= 0;
-            const float nx = (float)sm.sg[slot][0], ny = (float)sm.sg[slot][1], nz = (float)sm.sg[slot][2];
-            const float wsJ = (float)sm.sg[slot][3];
-            float qm[NS], qp[NS], Fm[NS], Fp[NS], wm, wp;
-            {
-                const float4 a4 = sm.auxa[PAD(vn)];
-                const float2 b2 = sm.auxb[PAD(vn)];
-                const float rho = 2.f * a4.x;
-                qm[0] = rho;
-                qm[1] = rho * (2.f * a4.y);
-                qm[2] = rho * (2.f * a4.z);
-                qm[3] = rho * (2.f * a4.w);
-                qm[4] = rho * (2.f * b2.x);
-            }
-            // normal flux and wave speed of one side (euler.jl:50-68)
-            auto side_flux = [&](const float (&qq)[NS], float (&F)[NS], float& w) {
-                const float rho = qq[0], rhoe = qq[4];
-                const float u0 = qq[1] / rho, u1 = qq[2] / rho, u2 = qq[3] / rho;
-                const float rr = qq[1] * qq[1] + qq[2] * qq[2] + qq[3] * qq[3];
-                const float p = gm1 * (rhoe - rr / (2.f * rho));
-                const float un = u0 * nx + u1 * ny + u2 * nz;
-                const float mn = qq[1] * nx + qq[2] * ny + qq[3] * nz;
-                F[0] = mn;
-                F[1] = mn * u0 + p * nx;
-                F[2] = mn * u1 + p * ny;
-                F[3] = mn * u2 + p * nz;
-                F[4] = un * (rhoe + p);
-                w = fabsf(un) + sqrtf(gam * p / rho);
-            };
-            side_flux(qm, Fm, wm);
-            if (open_face) {
-#pragma unroll
-                for (int s = 0; s < NS; ++s) qp[s] = (float)sm.slot[s][slot];
-                side_flux(qp, Fp, wp);
-            } else {  // boundary face: q+ = q- (balancelaw.jl:77)
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    qp[s] = qm[s];
-                    Fp[s] = Fm[s];
-                }
-                wp = wm;
-            }
-            const float mx = fmaxf(wm, wp);
-            const float mj = sm.mji[vn];
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const float fc = (Fm[s] + Fp[s]) * 0.5f;
-                const float nf = A.surface_rusanov ? fc - (mx * (qp[s] - qm[s])) * 0.5f : fc;
-                sm.slot[s][slot] = (double)((wsJ * nf) * mj);
-            }
-        }
-        // #2: face contributions ready, and the element's register has landed
-        if (__syncthreads_or(read_dq && !bounded_wait(&sm.bard, phd))) {
-            if (t == 0) atomicExch(A.status, kStatusTimeout);
-            return;
-        }
-        if (read_dq) phd ^= 1;
-        if (t == 0 && en < A.E) {  // the next element's face geometry (this element's faces are done)
+        if (t == 32) {
             fence_proxy_async();
-            mbar_expect_tx(&sm.bars, sgbytes);
-            bulk_g2s(&sm.sg[0][0], A.sgeo + (size_t)en * NSLOT * 4, sgbytes, &sm.bars);
+            fetch_rows(1, e);
+            fetch_rows(0, e);
         }
-        // ---- own nodes: dq = rka dq + volume - faces (x, y, z order); q_out = q + rkb dt dq
-        const size_t g0 = (size_t)e * NS * NP + t;
+        if (t == 64 && en < E) {
+            fence_proxy_async();
+            fetch_state(en);
+        }
+        if (t == 96 && reads_dq)  // the register, read at the element's end, into the L2 cache
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const T*>(A.dq) + (size_t)e * NS * NP),
+                         "n"(NS * NP * (int)sizeof(T))
+                         : "memory");
+        if (t < 6 && en < E) cp_async4(&sm.nb[buf ^ 1][t], A.nbr + (size_t)6 * en + t);
+        cp_async_commit();
+        const size_t g0 = (size_t)e * NS * NP;
+
+        // One direction: DIR, and POS 0 (writes its sums), 1 (adds to them), 2 (finishes)
+        auto direction = [&](auto dirc, auto posc) {
+            constexpr int DIR = decltype(dirc)::value, POS = decltype(posc)::value;
+            constexpr int STR = DIR == 0 ? 1 : DIR == 1 ? Q : Q * Q;
+            const line::HalfLine<Q, DIR> L(line::thread_index());
+            const int half = L.half, base = L.base;
+            const int end = base + (half ? (Q - 1) * STR : 0), step = half ? -STR : STR;
+            // ---- the neighbour's trace (q+ = q- on a boundary face, balancelaw.jl:77) and the face
+            // geometry at the thread's face node, before the pairs
+            const int f = 2 * DIR + half, nbf = sm.nb[buf][f];
+            double tr[NS], sg[4];
+            {
+                const double* qn = A.q_in + (nbf >= 0 ? (size_t)nbf * NS * NP + base + (half ? 0 : (Q - 1) * STR) : g0 + end);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int kk = k0 + 4 * h;
-            int slots[3] = {-1, -1, -1};
-            if (ii == 0) slots[0] = jj + 8 * kk;
-            else if (ii == NQ - 1) slots[0] = 64 + jj + 8 * kk;
-            if (jj == 0) slots[1] = 128 + ii + 8 * kk;
-            else if (jj == NQ - 1) slots[1] = 192 + ii + 8 * kk;
-            if (kk == 0) slots[2] = 256 + ii + 8 * jj;
-            else if (kk == NQ - 1) slots[2] = 320 + ii + 8 * jj;
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const size_t g = g0 + NT * h + s * NP;
-                float v = acc[h][s];
-                if (read_dq) v = (float)A.rka * sm.dqb[s][t + NT * h] + v;
+                for (int s = 0; s < NS; ++s) tr[s] = __ldg(qn + s * NP);
+                line::load4(A.sgeo + (((size_t)e * 6 + f) * NFP + L.jf) * 4, true, sg);
+            }
+            // ---- the line's rows, counted from the thread's end
+            late |= !bounded_wait(&sm.bar_geo[DIR], ph);
+            const double* const row = &sm.geo[3 * DIR][0];
+            T lo[H0][3], lf[H0][3];  // own nodes, the other half's
+            if constexpr (DIR == 0) {  // 4 consecutive nodes each
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
-                    if (slots[d] >= 0) v = v - (float)sm.slot[s][slots[d]];
-                A.dq[g] = v;
-                A.q_out[g] = __ldg(A.q_in + g) + A.rkb_dt * (double)v;
+#pragma unroll
+                    for (int far = 0; far < 2; ++far) {
+                        const double* r = row + d * NP + base + 4 * (far ? 1 - half : half);
+                        const double2 a = *reinterpret_cast<const double2*>(r), b = *reinterpret_cast<const double2*>(r + 2);
+                        const T v[4] = {(T)a.x, (T)a.y, (T)b.x, (T)b.y};
+#pragma unroll
+                        for (int m = 0; m < H0; ++m) (far ? lf : lo)[m][d] = half ? v[3 - m] : v[m];
+                    }
+            } else {
+#pragma unroll
+                for (int m = 0; m < H0; ++m)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) lo[m][d] = (T)row[d * NP + end + step * m];
             }
+            // ---- the partner values of the line's node a: see line_kernel.cuh
+            constexpr int S16 = DIR == 0 ? 1 : LS::slot16(STR), S8 = DIR > 0 ? STR / 2 : 1;
+            const int mid = end + (half ? -H0 : H0) * STR;
+            const int own16 = LS::slot16(end), own8 = LS::slot8(end), far16 = LS::slot16(mid), far8 = LS::slot8(mid);
+            auto values = [&](const int a, T (&v)[NAUX]) {
+                const int d = a < H0 ? a : a - H0;
+                if constexpr (DIR == 0)
+                    sm.aux.get(a < H0 ? own16 + d : far16 - d, a < H0 ? own8 ^ d : far8 ^ d, v);
+                else
+                    sm.aux.get((a < H0 ? own16 : far16) + (half ? -S16 : S16) * d,
+                               (a < H0 ? own8 : far8) + (half ? -S8 : S8) * d, v);
+            };
+            T acc[H0][NS], o[H0][NAUX];
+#pragma unroll
+            for (int m = 0; m < H0; ++m) {
+                values(m, o[m]);
+#pragma unroll
+                for (int s = 0; s < NS; ++s) acc[m][s] = T(0);
+            }
+#pragma unroll
+            for (int m = 0; m < H0; ++m)
+#pragma unroll
+                for (int n = m + 1; n < H0; ++n) {  // pairs of own nodes, once for both
+                    T G[3], un = T(0);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        G[d] = fma(pipec::dpar<T>(A, n, m), lo[n][d], -(pipec::dpar<T>(A, m, n) * lo[m][d]));
+                        un = fma(o[m][1 + d] + o[n][1 + d], G[d], un);
+                    }
+                    const T f1 = (o[m][0] + o[n][0]) * un, pb = o[m][5] + o[n][5];
+                    acc[m][0] += f1;
+                    acc[n][0] -= f1;
+#pragma unroll
+                    for (int c = 1; c < NS; ++c) {
+                        acc[m][c] = fma(f1, o[n][c], acc[m][c]);
+                        acc[n][c] = fma(-f1, o[m][c], acc[n][c]);
+                    }
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        acc[m][1 + d] = fma(pb, G[d], acc[m][1 + d]);
+                        acc[n][1 + d] = fma(-pb, G[d], acc[n][1 + d]);
+                    }
+                    acc[m][4] = fma(un, pb, acc[m][4]);
+                    acc[n][4] = fma(-un, pb, acc[n][4]);
+                }
+#pragma unroll
+            for (int a = H0; a < Q; ++a) {  // the other half's nodes
+                T p[NAUX], lp[3];
+                values(a, p);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) lp[d] = DIR == 0 ? lf[a - H0][d] : (T)row[d * NP + end + step * a];
+#pragma unroll
+                for (int m = 0; m < H0; ++m) {
+                    T G[3], un = T(0);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        G[d] = fma(pipec::dpar<T>(A, a, m), lp[d], -(pipec::dpar<T>(A, m, a) * lo[m][d]));
+                        un = fma(o[m][1 + d] + p[1 + d], G[d], un);
+                    }
+                    const T f1 = (o[m][0] + p[0]) * un, pb = o[m][5] + p[5];
+                    acc[m][0] += f1;
+#pragma unroll
+                    for (int c = 1; c < NS; ++c) acc[m][c] = fma(f1, p[c], acc[m][c]);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) acc[m][1 + d] = fma(pb, G[d], acc[m][1 + d]);
+                    acc[m][4] = fma(un, pb, acc[m][4]);
+                }
+            }
+            // the own-node parts of the averages, and the reflection of the far half
+#pragma unroll
+            for (int m = 0; m < H0; ++m) {
+#pragma unroll
+                for (int c = 1; c < NS; ++c) acc[m][c] = fma(o[m][c], acc[m][0], acc[m][c]);
+#pragma unroll
+                for (int s = 0; s < NS; ++s) acc[m][s] = half ? -acc[m][s] : acc[m][s];
+            }
+            // ---- face term at the thread's first node: wsJ nf (MJI follows at the end)
+            {
+                const T nv[3] = {(T)sg[0], (T)sg[1], (T)sg[2]}, wsJ = (T)sg[3];
+                const T rm = T(2) * o[0][0], pm = T(2) * o[0][5], Em = rm * (T(2) * o[0][4]);
+                const T rp = (T)tr[0], Ep = (T)tr[4], rinv = rcp(rp);
+                T um[3], mp[3], up[3], unm = T(0), unp = T(0);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    um[d] = T(2) * o[0][1 + d];
+                    mp[d] = (T)tr[1 + d];
+                    up[d] = mp[d] * rinv;
+                    unm = fma(um[d], nv[d], unm);
+                    unp = fma(up[d], nv[d], unp);
+                }
+                const T pp = pipec::gas<T>(A, 1) * (Ep - (mp[0] * mp[0] + mp[1] * mp[1] + mp[2] * mp[2]) * (T(0.5) * rinv));
+                // the larger wave speed |u.n| + sqrt(gamma p / rho) (euler.jl:62-68)
+                const T wm = fabs(unm) + root(pipec::gas<T>(A, 0) * pm * rcp(rm));
+                const T wp = fabs(unp) + root(pipec::gas<T>(A, 0) * pp * rinv);
+                const T mx = A.surface_rusanov ? fmax(wm, wp) : T(0);
+                const T mnm = rm * unm, mnp = rp * unp;
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    T fm, fp, dq;
+                    if (s == 0) {
+                        fm = mnm;
+                        fp = mnp;
+                        dq = rp - rm;
+                    } else if (s == 4) {
+                        fm = unm * (Em + pm);
+                        fp = unp * (Ep + pp);
+                        dq = Ep - Em;
+                    } else {
+                        fm = mnm * um[s - 1] + pm * nv[s - 1];
+                        fp = mnp * up[s - 1] + pp * nv[s - 1];
+                        dq = mp[s - 1] - rm * um[s - 1];
+                    }
+                    acc[0][s] -= wsJ * ((fm + fp) * T(0.5) - (mx * dq) * T(0.5));
+                }
+            }
+            // ---- hand the sums over, or finish: dq = rka dq + MJI sums; q_out = q + rkb dt dq
+            if constexpr (POS < 2) {
+#pragma unroll
+                for (int m = 0; m < H0; ++m) {
+                    const int n = LS::template sum_slot<T>(end + step * m);
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        if constexpr (POS == 0) sm.acc[s][n] = acc[m][s];
+                        else sm.acc[s][n] += acc[m][s];
+                    }
+                }
+            } else {
+                const int n0 = base + 4 * half;
+                const size_t g = line::after(g0 + n0);
+                const bool wide = (((uintptr_t)A.q_in | (uintptr_t)A.q_out | (sizeof(T) == 8 ? (uintptr_t)A.dq : 0)) & 31) == 0;
+                T mji[4];
+                {
+                    const double2 a = *reinterpret_cast<const double2*>(&sm.geo[9][n0]);
+                    const double2 b = *reinterpret_cast<const double2*>(&sm.geo[9][n0 + 2]);
+                    mji[0] = (T)a.x, mji[1] = (T)a.y, mji[2] = (T)b.x, mji[3] = (T)b.y;
+                }
+                double qold[NS][4];  // all loads before the stores, which might alias them
+                T old[NS][4];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    line::load4(A.q_in + g + s * NP, wide, qold[s]);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) old[s][m] = T(0);
+                    if (reads_dq) {
+                        if constexpr (sizeof(T) == 8) {
+                            line::load4(static_cast<const double*>(A.dq) + g + s * NP, wide, old[s]);
+                        } else {
+                            const float4 v = *reinterpret_cast<const float4*>(static_cast<const float*>(A.dq) + g + s * NP);
+                            old[s][0] = v.x, old[s][1] = v.y, old[s][2] = v.z, old[s][3] = v.w;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    T v[4];
+                    if constexpr (sizeof(T) == 8) {
+                        const double2 a = *reinterpret_cast<const double2*>(&sm.acc[s][LS::template sum_slot<T>(n0)]);
+                        const double2 b = *reinterpret_cast<const double2*>(&sm.acc[s][LS::template sum_slot<T>(n0 + 2)]);
+                        v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+                    } else {
+                        const float4 a = *reinterpret_cast<const float4*>(&sm.acc[s][LS::template sum_slot<T>(n0)]);
+                        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+                    }
+                    double out[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        v[m] += half ? acc[3 - m][s] : acc[m][s];
+                        v[m] = fma((T)A.rka, old[s][m], v[m] * mji[m]);
+                        out[m] = qold[s][m] + A.rkb_dt * (double)v[m];
+                    }
+                    if constexpr (sizeof(T) == 4)
+                        *reinterpret_cast<float4*>(static_cast<float*>(A.dq) + g + s * NP) = make_float4(v[0], v[1], v[2], v[3]);
+                    else
+                        line::store4(static_cast<double*>(A.dq) + g + s * NP, wide, v);
+                    line::store4(A.q_out + g + s * NP, wide, out);
+                }
+            }
+        };
+        using I0 = std::integral_constant<int, 0>;
+        using I1 = std::integral_constant<int, 1>;
+        using I2 = std::integral_constant<int, 2>;
+        direction(I2{}, I0{});
+        __syncthreads();  // #2: the z sums of the warp's planes; the z rows are free
+        if (t == 96 && en < E) {
+            fence_proxy_async();
+            fetch_rows(2, en);
         }
+        direction(I1{}, I1{});
+        __syncwarp();
+        direction(I0{}, I2{});
     }
+    if (late) atomicExch(A.status, kStatusTimeout);  // the last element's rows
 }
 
 }  // namespace rb200

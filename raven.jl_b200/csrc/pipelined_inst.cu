@@ -3,7 +3,6 @@
 // state (the DGSEM handle) or the chunks of a serving class (BATCH).
 #include "pipelined_adv.cuh"
 #include "pipelined_curved.cuh"
-#include "pipelined_curved64.cuh"
 #include "pipelined_kernel.cuh"
 
 namespace rb200 {
@@ -97,46 +96,27 @@ int pipelined_batch_blocks_per_sm(int nq, int combo, int fp32) {
     return fp32 ? occupancy_adv<float, true>(nq) : occupancy_adv<double, true>(nq);
 }
 
-// The curved-grid kernel (FP32 bulk, Kennedy-Gruber): two CTAs per SM.
-cudaError_t launch_pipelined_curved(const PipeCurvedArgs& a, int grid, cudaStream_t s) {
-    auto kern = pipelined_curved_kernel<EUL_KG>;
+// The curved-grid kernel (Kennedy-Gruber).  blocks_per_sm != nullptr: occupancy query only.
+template <typename T>
+static cudaError_t launch_c(const PipeCurvedArgs& a, int grid, cudaStream_t s, int* blocks_per_sm) {
+    auto kern = pipelined_curved_kernel<T>;
+    constexpr size_t smem = sizeof(pipec::Smem<T>);
     static std::atomic<uint64_t> configured{0};
-    cudaError_t err = ensure_smem_limit(kern, (int)sizeof(pipec::Smem), configured);
+    cudaError_t err = ensure_smem_limit(kern, (int)smem, configured);
     if (err != cudaSuccess) return err;
-    kern<<<grid, pipec::NT, sizeof(pipec::Smem), s>>>(a);
+    if (blocks_per_sm) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, pipec::NT, smem);
+    kern<<<grid, pipec::NT, smem, s>>>(a);
     return cudaGetLastError();
 }
 
-// The curved-grid kernel in FP64 (Kennedy-Gruber): two CTAs per SM.
-cudaError_t launch_pipelined_curved64(const PipeCurvedArgs& a, int grid, cudaStream_t s) {
-    auto kern = pipelined_curved64_kernel<EUL_KG>;
-    static std::atomic<uint64_t> configured{0};
-    cudaError_t err = ensure_smem_limit(kern, (int)sizeof(pipec64::Smem), configured);
-    if (err != cudaSuccess) return err;
-    kern<<<grid, pipec64::NT, sizeof(pipec64::Smem), s>>>(a);
-    return cudaGetLastError();
+cudaError_t launch_pipelined_curved(int fp32, const PipeCurvedArgs& a, int grid, cudaStream_t s) {
+    return fp32 ? launch_c<float>(a, grid, s, nullptr) : launch_c<double>(a, grid, s, nullptr);
 }
 
-int pipelined_curved64_blocks_per_sm() {
-    auto kern = pipelined_curved64_kernel<EUL_KG>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(pipec64::Smem)) !=
-        cudaSuccess)
-        return 0;
+int pipelined_curved_blocks_per_sm(int fp32) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, pipec64::NT, sizeof(pipec64::Smem)) != cudaSuccess)
-        return 0;
-    return n;
-}
-
-int pipelined_curved_blocks_per_sm() {
-    auto kern = pipelined_curved_kernel<EUL_KG>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(pipec::Smem)) !=
-        cudaSuccess)
-        return 0;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, pipec::NT, sizeof(pipec::Smem)) != cudaSuccess)
-        return 0;
-    return n;
+    const PipeCurvedArgs none{};
+    return (fp32 ? launch_c<float>(none, 0, nullptr, &n) : launch_c<double>(none, 0, nullptr, &n)) == cudaSuccess ? n : 0;
 }
 
 }  // namespace rb200

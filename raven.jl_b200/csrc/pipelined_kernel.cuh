@@ -82,6 +82,15 @@ inline bool pipe_tables(PipeArgs& p, int combo, int nq, double gamma, const doub
     return odd;
 }
 
+// Whether D is odd under reflection of the line, to 8 roundings (every Lobatto line's is).
+inline bool pipe_odd_derivative(int nq, const double* D) {
+    double big = 0.0;
+    for (int i = 0; i < nq * nq; ++i) big = std::max(big, std::fabs(D[i]));
+    bool odd = true;
+    for (int i = 0; i < nq * nq; ++i) odd = odd && std::fabs(D[i] + D[nq * nq - 1 - i]) <= 8 * 2.220446049250313e-16 * big;
+    return odd;
+}
+
 // Serving loop: the elements of a launch are the chunks of a class's running solves
 // instead of the strided elements of one state (SolveDesc, Chunk: rb200_internal.h).
 struct PipeBatch {

@@ -195,12 +195,9 @@ cudaError_t launch_pipelined_batch(int nq, int combo, int fp32, const PipeArgs& 
                                    cudaStream_t s);
 int pipelined_batch_blocks_per_sm(int nq, int combo, int fp32);
 struct PipeCurvedArgs;  // pipelined_curved.cuh
-// Persistent pipelined kernel for 3-D Nq = 8 curved grids (FP32 bulk, Kennedy-Gruber, stage modes).
-cudaError_t launch_pipelined_curved(const PipeCurvedArgs& a, int grid, cudaStream_t s);
-int pipelined_curved_blocks_per_sm();
-// The same in FP64 (Kennedy-Gruber, stage modes).
-cudaError_t launch_pipelined_curved64(const PipeCurvedArgs& a, int grid, cudaStream_t s);
-int pipelined_curved64_blocks_per_sm();
+// Persistent pipelined kernel for 3-D Nq = 8 curved grids (Kennedy-Gruber, stage modes).
+cudaError_t launch_pipelined_curved(int fp32, const PipeCurvedArgs& a, int grid, cudaStream_t s);
+int pipelined_curved_blocks_per_sm(int fp32);
 
 // Reductions and face-map expansion (reduce.cu).
 cudaError_t launch_weighted_sums(const double* q, const double* elem_geo, const double* vgeo, const double* w,

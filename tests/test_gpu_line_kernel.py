@@ -1,5 +1,5 @@
 """The half-line stage kernel of 3-D Euler on unwarped bricks (Nq = 4..8; Kennedy-Gruber,
-entropy conservative, central flux differencing and the weak form) against the oracle and
+entropy conservative, central flux differencing and the weak form), and its curved form, against the oracle and
 the generic stage kernel: grids with fewer and with more elements than its CTAs, faces on
 the boundary, tendencies that set and that add, and buffers aligned to 16 bytes only.
 
@@ -98,3 +98,29 @@ def test_sixteen_byte_alignment(rb, cuda_ok, nq):
     dg.sync_status()
     assert torch.equal(aligned.data, moved.data) and torch.equal(a.dq.data, b.dq.data)
     assert np.isfinite(aligned.numpy()).all()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_bulk"])
+def test_curved_sixteen_byte_alignment(rb, cuda_ok, precision):
+    """The curved kernel (Nq = 8) on open faces with a state 16 bytes past a 32-byte boundary:
+    the same bits as an aligned one, and the generic kernel's state to 1e-12 (FP32 bulk 1e-6)."""
+    import torch
+
+    og = O.Grid(3, 8, (2, 3, 2), [0.0] * 3, [10.0] * 3, (1, 0, 1), O.WARP_SINE, 0.1)
+    law, form = product_scheme(rb, "eul_kg", 3)
+    dg = rb.DGSEM(law=law, grid=wrap_oracle_grid(og), volume_form=form, surface_numericalflux=rb.RusanovFlux(),
+                  precision=precision)
+    assert dg.geometry == "curved" and dg.pipelined_ctas > 0
+    q = initial_state(og, oracle_law("eul_kg", 3), "eul_kg", seed=6)
+    a = rb.GridArray.from_numpy(q)
+    t = torch.empty(a.data.numel() + 2, dtype=a.data.dtype, device=a.data.device)[2:].view(a.data.shape)
+    assert t.data_ptr() % 32 == 16
+    b = rb.GridArray(t.copy_(a.data), a.ns, a.np, a.E)
+    for x in (a, b):
+        rb.LSRK54(dg, x, 1e-3).dostep(x, 2)
+    dg.sync_status()
+    assert torch.equal(a.data, b.data)
+    dg.set_kernel_path("generic")
+    c = rb.GridArray.from_numpy(q)
+    rb.LSRK54(dg, c, 1e-3).dostep(c, 2)
+    assert rel_err(a.numpy(), c.numpy()) <= (1e-12 if precision == "fp64" else 1e-6)
