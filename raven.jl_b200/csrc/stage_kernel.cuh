@@ -98,9 +98,6 @@ struct Prefetched {
     bool tables_ready = false;
 };
 
-__device__ __forceinline__ double dev_sqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ float dev_sqrt(float x) { return sqrtf(x); }
-
 // Buffers of the element being updated: the DGSEM handle takes them from StageArgs,
 // the serving loop from each solve's descriptor.
 struct ElemPtrs {
@@ -288,7 +285,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
             for (int d = 1; d < DIM; ++d) wJ = wJ * A.w[id[d]];
             wJ = wJ * J;
-            mji = 1.0 / wJ;
+            mji = rcp(wJ);
 #pragma unroll
             for (int d = 0; d < DIM; ++d) lg[d] = (T)(wJ * drdx[d]);
         } else {
@@ -321,25 +318,26 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
         } else {
             const T rho = q[0];
             const T rhoe = q[DIM + 1];
+            const T rinv = rcp(rho);
             T u[DIM];
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) u[d] = q[1 + d] / rho;
+            for (int d = 0; d < DIM; ++d) u[d] = q[1 + d] * rinv;
             T rr = q[1] * q[1];
 #pragma unroll
             for (int d = 1; d < DIM; ++d) rr = rr + q[1 + d] * q[1 + d];
             const T gm1 = (T)(A.gamma - 1.0);
-            const T p = gm1 * (rhoe - rr / (T(2) * rho));
+            const T p = gm1 * (rhoe - rr * (T(0.5) * rinv));
             if constexpr (COMBO == EUL_KG) {
                 own[0] = rho * T(0.5);
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) own[1 + d] = u[d] * T(0.5);
-                own[DIM + 1] = (rhoe / rho) * T(0.5);
+                own[DIM + 1] = (rhoe * rinv) * T(0.5);
                 own[DIM + 2] = p * T(0.5);
             } else if constexpr (COMBO == EUL_EC) {
                 own[0] = rho;
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) own[1 + d] = u[d];
-                own[DIM + 1] = rho / (T(2) * p);
+                own[DIM + 1] = T(0.5) * rho * rcp(p);
                 T uu = u[0] * u[0];
 #pragma unroll
                 for (int d = 1; d < DIM; ++d) uu = uu + u[d] * u[d];
@@ -628,14 +626,14 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
                 for (int side2 = 0; side2 < 2; ++side2) {
                     const T* qq = side2 == 0 ? q : qp;
-                    const T rho = qq[0], rhoe = qq[DIM + 1];
+                    const T rho = qq[0], rhoe = qq[DIM + 1], rinv = rcp(rho);
                     T u[DIM];
 #pragma unroll
-                    for (int d = 0; d < DIM; ++d) u[d] = qq[1 + d] / rho;
+                    for (int d = 0; d < DIM; ++d) u[d] = qq[1 + d] * rinv;
                     T rr = qq[1] * qq[1];
 #pragma unroll
                     for (int d = 1; d < DIM; ++d) rr = rr + qq[1 + d] * qq[1 + d];
-                    const T p = gm1 * (rhoe - rr / (T(2) * rho));
+                    const T p = gm1 * (rhoe - rr * (T(0.5) * rinv));
                     T un, mn;
                     if constexpr (AFF) {
                         un = u[dir] * nv[dir];
@@ -653,7 +651,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
                     for (int b = 0; b < DIM; ++b) Fn[side2][1 + b] = mn * u[b] + p * nv[b];
                     Fn[side2][DIM + 1] = un * (rhoe + p);
-                    ws[side2] = fabs(un) + dev_sqrt((T)A.gamma * p / rho);
+                    ws[side2] = fabs(un) + root((T)A.gamma * p * rinv);
                 }
                 const T mx = fmax(ws[0], ws[1]);
 #pragma unroll
@@ -717,6 +715,9 @@ __global__ void __launch_bounds__(Shape<DIM, NQ>::THREADS, (PersistentCfg<DIM, N
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using S = Shape<DIM, NQ>;
     using PC = PersistentCfg<DIM, NQ, COMBO, GEOM, T>;
+    // launched while the previous kernel of the stream drains, as the pipelined kernels are: a
+    // stage of a small grid is mostly launch latency
+    grid_dependency_wait();
     if constexpr (!PC::PF) {
         const int64_t e = A.e_begin + (int64_t)blockIdx.x * S::EPB + threadIdx.x / S::NP;
         stage_element<DIM, NQ, COMBO, GEOM, T, 0, SF>(A, elem_ptrs(A), e, e < A.E, smem_raw);
@@ -772,8 +773,7 @@ cudaError_t launch_one(const StageArgs& a, cudaStream_t st) {
     const int64_t groups = (a.E - a.e_begin + S::EPB - 1) / S::EPB;
     if (groups <= 0) return cudaSuccess;
     if constexpr (!PC::PF) {
-        kern<<<(unsigned)groups, S::THREADS, PC::smem, st>>>(a);
-        return cudaGetLastError();
+        return launch_pdl(kern, (int)groups, S::THREADS, PC::smem, st, a);
     }
     // persistent grid: the resident CTAs of every SM, cached per device
     static std::atomic<int> grid_of_device[64];
@@ -788,8 +788,7 @@ cudaError_t launch_one(const StageArgs& a, cudaStream_t st) {
         grid = per_sm > 0 ? per_sm * nsm : 1;
         if (dev >= 0 && dev < 64) grid_of_device[dev].store(grid, std::memory_order_relaxed);
     }
-    kern<<<(unsigned)std::min<int64_t>(grid, groups), S::THREADS, PC::smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(kern, (int)std::min<int64_t>(grid, groups), S::THREADS, PC::smem, st, a);
 }
 
 // Small grids: every stage of every step of an LSRK call in one launch of one
