@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(Q * Q * Q / pipea::npt<Q>(), (pipe_adv_min_cta
     const bool dq_is_f32 = stage && sizeof(T) == 4;
     // the register arrives by bulk copy whenever the stage reads it in type T
     const bool bulk_dq = A.mode == MODE_STAGE || (A.mode == MODE_TENDENCY_INC && sizeof(T) == 8);
+    // the previous kernel of the stream (the last stage, or this stage's mortar fluxes) is complete
+    grid_dependency_wait();
     const uint32_t qbytes = NP * sizeof(double), dqbytes = bulk_dq ? NP * sizeof(T) : 0;
 
     // Threads 0..9 put element `r` into ring stage `s`: thread 0 the bulk copies of its

@@ -106,12 +106,11 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
 #pragma unroll
         for (int d = 0; d < 3; ++d) mbar_init(&sm.bar_geo[d], 1);
         fence_mbar_init();
-        if (e < E) {
-            fetch_rows(2, e);  // geometry: written by no kernel
-            fetch_state(e);
-        }
+        if (e < E) fetch_rows(2, e);  // geometry: written by no kernel
     }
     if (t < 6 && e < E) cp_async4(&sm.nb[0][t], A.nbr + (size_t)6 * e + t);
+    grid_dependency_wait();  // the previous kernel of the stream is complete
+    if (t == 0 && e < E) fetch_state(e);
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();

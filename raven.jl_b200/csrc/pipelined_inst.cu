@@ -32,6 +32,9 @@ static cudaError_t launch_a(const PipeArgs& a, const PipeBatch& b, int grid, cud
     static std::atomic<uint64_t> configured{0};
     cudaError_t err = ensure_smem_limit(kern, (int)sizeof(pipea::Smem<T, Q>), configured);
     if (err != cudaSuccess) return err;
+    // (a serving tick's first stage follows host-written chunk tables: plain order)
+    if (!BATCH || b.stage > 0)
+        return launch_pdl(kern, grid, Q * Q * Q / pipea::npt<Q>(), sizeof(pipea::Smem<T, Q>), s, a, b);
     kern<<<grid, Q * Q * Q / pipea::npt<Q>(), sizeof(pipea::Smem<T, Q>), s>>>(a, b);
     return cudaGetLastError();
 }
@@ -105,8 +108,7 @@ static cudaError_t launch_c(const PipeCurvedArgs& a, int grid, cudaStream_t s, i
     cudaError_t err = ensure_smem_limit(kern, (int)smem, configured);
     if (err != cudaSuccess) return err;
     if (blocks_per_sm) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, pipec::NT, smem);
-    kern<<<grid, pipec::NT, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, pipec::NT, smem, s, a);
 }
 
 cudaError_t launch_pipelined_curved(int fp32, const PipeCurvedArgs& a, int grid, cudaStream_t s) {
