@@ -322,7 +322,7 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
     if (e != cudaSuccess) return e;
     c.ntiles = c.dim == 2 ? batched_tiles_d2(c.nq, c.epb) : batched_tiles_d3(c.nq, c.epb);
     if (c.ntiles <= 0) return cudaErrorInvalidValue;
-    // a chunk is 8 default tiles: a multiple of every candidate tile
+    // a chunk is at most 8 default tiles (see launch_ticks)
     c.chunk_elems = 8 * c.epb[1];
     int nsm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device);
