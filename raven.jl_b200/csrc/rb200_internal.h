@@ -186,11 +186,12 @@ cudaError_t launch_stage(int dim, int nq, int combo, int geom, int fp32, const S
 size_t stage_smem_bytes(int dim, int nq, int combo, int geom, int fp32);
 
 struct PipeArgs;  // pipelined_kernel.cuh
-// Persistent TMA-pipelined kernel for 3-D Nq = 8 affine flux differencing (KG, EC).
+// Persistent kernels of 3-D unwarped bricks: Euler (half lines, Nq = 4..8) and weak-form advection
+// (Nq = 4, 6, 8).
 cudaError_t launch_pipelined(int nq, int combo, int fp32, const PipeArgs& a, int grid, cudaStream_t s);
 int pipelined_blocks_per_sm(int nq, int combo, int fp32);
 struct PipeBatch;  // pipelined_kernel.cuh
-// The same kernel over the chunks of a serving class (Euler KG only).
+// The same kernels over the chunks of a serving class (Euler KG or advection, even Nq).
 cudaError_t launch_pipelined_batch(int nq, int combo, int fp32, const PipeArgs& a, const PipeBatch& b, int grid,
                                    cudaStream_t s);
 int pipelined_batch_blocks_per_sm(int nq, int combo, int fp32);
