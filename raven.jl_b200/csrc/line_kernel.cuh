@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
             sn = NFP;
         }
 #pragma unroll
-        for (int s = 0; s < NS; ++s) tr[DIR][s] = __ldg(qn + s * sn);
+        for (int s = 0; s < NS; ++s) tr[DIR][s] = qn[s * sn];
     };
     using I0 = std::integral_constant<int, 0>;
     using I1 = std::integral_constant<int, 1>;

@@ -170,18 +170,23 @@ __global__ void __launch_bounds__((DIM == 3 ? 4 : 2) * Pow<NQ, DIM - 1>::v)
         const int64_t eC = col[0];
         const int fC = (int)col[1], fF = fC ^ 1, dir = fC >> 1;
         const T sn = (fC & 1) ? T(1) : T(-1);
+        const int64_t eF = col[2 + k];
+        T qf[NS];  // the small face's trace, under way with the large one's
+        {
+            const int v = face_vol_node<DIM, NQ>(fF, j);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) qf[s] = (T)A.q[((size_t)eF * NS + s) * NP + v];
+        }
         if (t < NFP) {
             const int v = face_vol_node<DIM, NQ>(fC, t);
 #pragma unroll
-            for (int s = 0; s < NS; ++s) qC[s][t] = (T)__ldg(A.q + ((size_t)eC * NS + s) * NP + v);
+            for (int s = 0; s < NS; ++s) qC[s][t] = (T)A.q[((size_t)eC * NS + s) * NP + v];
         }
         __syncthreads();
         {
-            const int64_t eF = col[2 + k];
             const double* Ia = (k & 1) ? A.IU : A.IL;
             const double* Ib = (k >> 1) ? A.IU : A.IL;
-            T qi[NS], qf[NS], nf[NS];
-            const int v = face_vol_node<DIM, NQ>(fF, j);
+            T qi[NS], nf[NS];
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 T acc = T(0);
@@ -193,7 +198,6 @@ __global__ void __launch_bounds__((DIM == 3 ? 4 : 2) * Pow<NQ, DIM - 1>::v)
                     acc = fma(DIM == 3 ? (T)Ib[j2 * NQ + b] : T(1), tt, acc);
                 }
                 qi[s] = acc;
-                qf[s] = (T)__ldg(A.q + ((size_t)eF * NS + s) * NP + v);
             }
             if (A.sgeo) {
                 // curved: the small face's own normal, flipped to point out of the large

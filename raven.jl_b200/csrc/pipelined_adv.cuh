@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(Q * Q * Q / pipea::npt<Q>(), (pipe_adv_min_cta
             if (A.mode == MODE_STAGE) {
                 v = (T)A.rka * sm.dq[r][n] + v;
             } else if (A.mode == MODE_TENDENCY_INC) {
-                const double old = bulk_dq ? (double)sm.dq[r][n] : __ldg(reinterpret_cast<const double*>(dq_e) + g);
+                const double old = bulk_dq ? (double)sm.dq[r][n] : reinterpret_cast<const double*>(dq_e)[g];
                 v = (T)(old + (double)v);
             }
             if (ii == 0) v = v - (T)fl[jj + Q * kk];

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
             {
                 const double* qn = A.q_in + (nbf >= 0 ? (size_t)nbf * NS * NP + base + (half ? 0 : (Q - 1) * STR) : g0 + end);
 #pragma unroll
-                for (int s = 0; s < NS; ++s) tr[s] = __ldg(qn + s * NP);
+                for (int s = 0; s < NS; ++s) tr[s] = qn[s * NP];
                 line::load4(A.sgeo + (((size_t)e * 6 + f) * NFP + L.jf) * 4, true, sg);
             }
             // ---- the line's rows, counted from the thread's end

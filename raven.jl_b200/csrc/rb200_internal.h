@@ -88,7 +88,10 @@ struct StageArgs {
 // may start while the previous kernel of the stream drains; it touches no global memory
 // that kernel writes or reads before grid_dependency_wait() (griddepcontrol.wait: the
 // previous grid has completed and its writes are visible; a no-op in a kernel launched
-// without it).  RB200_PDL=0 launches the kernels in plain stream order.
+// without it).  States, registers and mortar fluxes are therefore read by ordinary loads or copies, which
+// stay behind that wait: __ldg is for what no kernel of the stream writes (geometry and
+// connectivity), since it promises data that is constant while the kernel is resident, and the
+// compiler may move it above the wait.  RB200_PDL=0 launches the kernels in plain stream order.
 #ifndef RB200_PDL
 #define RB200_PDL 1
 #endif

@@ -141,7 +141,7 @@ __device__ __forceinline__ void stage_element_adv_brick(const StageArgs& A, cons
     double qd = 0.0, drdx[3] = {0.0, 0.0, 0.0};
     T q0 = T(0);
     if (active) {
-        qd = pf.q ? pf.q[0] : __ldg(P.q_in + (size_t)e * NP + n);
+        qd = pf.q ? pf.q[0] : P.q_in[(size_t)e * NP + n];
         q0 = (T)qd;
         const double* eg = P.elem_geo + 4 * e;
 #pragma unroll
@@ -202,12 +202,12 @@ __device__ __forceinline__ void stage_element_adv_brick(const StageArgs& A, cons
             if (DIM == 1) j = 0;
             else if (DIM == 2) j = (dir == 0) ? id[1] : id[0];
             else j = (dir == 0) ? id[1] + NQ * id[2] : (dir == 1 ? id[0] + NQ * id[2] : id[0] + NQ * id[1]);
-            nf = (T)__ldg(P.ncflux + ((size_t)e * NF + f) * NFP + j);
+            nf = (T)P.ncflux[((size_t)e * NF + f) * NFP + j];
         } else {
             T qp = q0;  // default boundarystate (balancelaw.jl:77)
             if (ne >= 0) {
                 const int nn = n + (side == 0 ? (NQ - 1) * stride : -(NQ - 1) * stride);
-                qp = (T)__ldg(P.q_in + (size_t)ne * NP + nn);
+                qp = (T)P.q_in[(size_t)ne * NP + nn];
             } else if (ne <= -kBcBase && A.bc_kind[-ne - kBcBase] == BC_PRESCRIBED) {
                 qp = (T)A.bc_state[-ne - kBcBase][0];
             }
@@ -272,7 +272,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
         const double* qe = P.q_in + (size_t)e * NS * NP;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            qd[s] = pf.q ? pf.q[s * pf.stride] : __ldg(qe + s * NP + n);
+            qd[s] = pf.q ? pf.q[s * pf.stride] : qe[s * NP + n];
             q[s] = (T)qd[s];
         }
         if constexpr (AFF) {
@@ -560,7 +560,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
                     qn = P.q_in + (size_t)ne * NS * NP + nn;
                 }
 #pragma unroll
-                for (int s = 0; s < NS; ++s) qp[s] = (T)__ldg(qn + s * NP);
+                for (int s = 0; s < NS; ++s) qp[s] = (T)qn[s * NP];
             } else {
 #pragma unroll
                 for (int s = 0; s < NS; ++s) qp[s] = q[s];  // default boundarystate (balancelaw.jl:77)
@@ -605,7 +605,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
             T nf[NS];
             if (ne == -2) {  // mortar face of an adapted grid: the flux comes from the mortar kernel
 #pragma unroll
-                for (int s = 0; s < NS; ++s) nf[s] = (T)__ldg(P.ncflux + (((size_t)e * NF + f) * NS + s) * NFP + j);
+                for (int s = 0; s < NS; ++s) nf[s] = (T)P.ncflux[(((size_t)e * NF + f) * NS + s) * NFP + j];
             } else if constexpr (SF == 1 && !C::ADV) {
                 euler_entropy_surface_flux<DIM, T>(A.surface_flux, nv, q, qp, (T)A.gamma, nf);
             } else if constexpr (C::ADV) {
