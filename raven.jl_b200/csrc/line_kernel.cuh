@@ -225,6 +225,9 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
         if (t == 0) atomicExch(A.status, kStatusTimeout);
         return true;
     };
+    auto pressure = [&](const T rinv, const T m0, const T m1, const T m2, const T E) {
+        return line::gas<T>(A, 1) * (E - (m0 * m0 + m1 * m1 + m2 * m2) * (T(0.5) * rinv));
+    };
     // the state of element r: a bulk copy by thread 0, or each thread its own values
     auto fetch_state = [&](const double* q, int64_t e, int b) {
         const double* src = q + (size_t)e * NS * NP;
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 const T m0 = (T)sm.q[buf][1][n], m1 = (T)sm.q[buf][2][n], m2 = (T)sm.q[buf][3][n];
                 const T u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
                 const T rhoe = (T)sm.q[buf][4][n];
-                const T p = line::gas<T>(A, 1) * (rhoe - (m0 * m0 + m1 * m1 + m2 * m2) * (T(0.5) * rinv));
+                const T p = pressure(rinv, m0, m1, m2, rhoe);
                 T o[NAUX];
                 if constexpr (COMBO == EUL_KG) {  // halves of rho, u, e, p
                     o[0] = rho * T(0.5);
@@ -553,23 +556,19 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
             {
                 const T fsc = (T)(fabs(drdx) * A.winv[0]);
                 const T sn = half ? T(1) : T(-1);
-                // q- and its primitives from the partner values of the node
-                T rm, um[3], pm, Em;
-                if constexpr (COMBO == EUL_KG) {
-                    rm = T(2) * o[0][0];
-                    pm = T(2) * o[0][5];
-                    Em = rm * (T(2) * o[0][4]);
-                } else if constexpr (COMBO == EUL_EC) {
-                    rm = o[0][0];
-                    pm = rm * (T(0.5) * rcp(o[0][4]));
-                    Em = pm * (T(2) * line::gas<T>(A, 2)) + T(0.5) * rm * o[0][5];
-                } else {
-                    rm = o[0][0];
-                    pm = o[0][5];
-                    Em = o[0][4];
-                }
+                // q- is the state itself, and its velocity and pressure are what the element across
+                // the face takes from it: both compute the same flux, and equal states (q+ is q- on
+                // a boundary face) have no jump
+                T qm[NS], um[3], pm;
+#pragma unroll
+                for (int s = 1; s < NS; ++s)
+                    qm[s] = s == 4 && COMBO == EUL_WEAK ? o[0][4] : (T)sm.q[buf][s][end];
+                const T rm = qm[0] = COMBO == EUL_KG ? T(2) * o[0][0] : o[0][0], rmi = rcp(rm);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) um[d] = COMBO == EUL_KG ? T(2) * o[0][1 + d] : o[0][1 + d];
+                if constexpr (COMBO == EUL_KG) pm = T(2) * o[0][5];
+                else if constexpr (COMBO == EUL_WEAK) pm = o[0][5];
+                else pm = pressure(rmi, qm[1], qm[2], qm[3], qm[4]);
                 const T rp = (T)tr[DIR][0], Ep = (T)tr[DIR][4], rinv = rcp(rp);
                 T mp[3], up[3];
 #pragma unroll
@@ -577,10 +576,10 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                     mp[d] = (T)tr[DIR][1 + d];
                     up[d] = mp[d] * rinv;
                 }
-                const T pp = line::gas<T>(A, 1) * (Ep - (mp[0] * mp[0] + mp[1] * mp[1] + mp[2] * mp[2]) * (T(0.5) * rinv));
-                const T unm = um[DIR] * sn, unp = up[DIR] * sn, mnm = rm * unm, mnp = mp[DIR] * sn;
+                const T pp = pressure(rinv, mp[0], mp[1], mp[2], Ep);
+                const T unm = um[DIR] * sn, unp = up[DIR] * sn, mnm = qm[1 + DIR] * sn, mnp = mp[DIR] * sn;
                 // the larger wave speed |u.n| + sqrt(gamma p / rho) (euler.jl:62-68)
-                const T wm = fabs(unm) + root(line::gas<T>(A, 0) * pm * rcp(rm)), wp = fabs(unp) + root(line::gas<T>(A, 0) * pp * rinv);
+                const T wm = fabs(unm) + root(line::gas<T>(A, 0) * pm * rmi), wp = fabs(unp) + root(line::gas<T>(A, 0) * pp * rinv);
                 const T mx = A.surface_rusanov ? fmax(wm, wp) : T(0);
                 // normal fluxes of both sides (euler.jl:50-60 with n = sn e_dir), field by field
 #pragma unroll
@@ -591,13 +590,13 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                         fp = mnp;
                         dq = rp - rm;
                     } else if (s == 4) {
-                        fm = unm * (Em + pm);
+                        fm = unm * (qm[4] + pm);
                         fp = unp * (Ep + pp);
-                        dq = Ep - Em;
+                        dq = Ep - qm[4];
                     } else {
                         fm = mnm * um[s - 1] + (DIR == s - 1 ? pm * sn : T(0));
                         fp = mnp * up[s - 1] + (DIR == s - 1 ? pp * sn : T(0));
-                        dq = mp[s - 1] - rm * um[s - 1];
+                        dq = mp[s - 1] - qm[s];
                     }
                     const T nf = (fm + fp) * T(0.5) - (mx * dq) * T(0.5);
                     acc[0][s] -= (mortar[DIR] ? (T)tr[DIR][s] : nf) * fsc;

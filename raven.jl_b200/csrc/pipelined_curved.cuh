@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
                 // the larger wave speed |u.n| + sqrt(gamma p / rho) (euler.jl:62-68)
                 const T wm = fabs(unm) + root(pipec::gas<T>(A, 0) * pm * rcp(rm));
                 const T wp = fabs(unp) + root(pipec::gas<T>(A, 0) * pp * rinv);
-                const T mx = A.surface_rusanov ? fmax(wm, wp) : T(0);
+                // (q+ is q- on a boundary face: no jump, whatever the primitives' rounding)
+                const T mx = A.surface_rusanov && nbf >= 0 ? fmax(wm, wp) : T(0);
                 const T mnm = rm * unm, mnp = rp * unp;
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {

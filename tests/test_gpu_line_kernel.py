@@ -124,3 +124,56 @@ def test_curved_sixteen_byte_alignment(rb, cuda_ok, precision):
     c = rb.GridArray.from_numpy(q)
     rb.LSRK54(dg, c, 1e-3).dostep(c, 2)
     assert rel_err(a.numpy(), c.numpy()) <= (1e-12 if precision == "fp64" else 1e-6)
+
+
+def _continuous_state(og, seed):
+    """A state whose values at a point are the same bits in every element that has it."""
+    x = np.moveaxis(og.points(), 1, 2).reshape(-1, 3)  # (np * E, 3)
+    key = np.round(np.mod(x / np.array([10.0, 8.0, 9.0]), 1.0) * 1e6).astype(np.int64) % 10**6
+    _, point = np.unique(key, axis=0, return_inverse=True)
+    r = np.random.default_rng(seed).uniform(-0.1, 0.1, (5, point.max() + 1))[:, point.ravel()]
+    rho, u = 1 + r[0], [0.4 + r[1], -0.3 + r[2], 0.2 + r[3]]
+    E = (0.7 + r[4]) / 0.4 + rho * sum(v * v for v in u) / 2
+    return np.asfortranarray(np.stack([rho] + [rho * v for v in u] + [E]).reshape(5, og.np, og.E).transpose(1, 0, 2))
+
+
+@pytest.mark.parametrize("nq", range(4, 9))
+@pytest.mark.parametrize("scheme", SCHEMES)
+def test_equal_traces_have_no_jump(rb, cuda_ok, scheme, nq):
+    """On a state that is continuous across the faces, and at open faces, q+ - q- is exactly 0:
+    Rusanov and central faces give the same bits, in tendencies and in both precisions' steps."""
+    og = O.Grid(3, nq, (3, 2, 2), [0.0] * 3, [10.0, 8.0, 9.0], (1, 0, 1))
+    q = _continuous_state(og, 8)
+    law, form = product_scheme(rb, scheme, 3)
+    for precision in ("fp64", "fp32_bulk"):
+        out = []
+        for flux in (rb.RusanovFlux(), rb.CentralFlux()):
+            dg = rb.DGSEM(law=law, grid=wrap_oracle_grid(og), volume_form=form, surface_numericalflux=flux,
+                          precision=precision)
+            assert dg.pipelined_ctas > 0
+            qg = rb.GridArray.from_numpy(q)
+            dq = qg.similar()
+            dg(dq, qg, 0.0, increment=False)
+            q_out = qg.similar()
+            dg.lsrk54_stage(qg, q_out, qg.similar(), 0, 0.0, 1e-3)
+            out.append((dq.numpy(), q_out.numpy()))
+        assert np.array_equal(out[0][0], out[1][0])
+        assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_bulk"])
+def test_curved_open_faces_have_no_jump(rb, cuda_ok, precision):
+    """One element with six open faces on the curved kernel: Rusanov and central faces alike."""
+    og = O.Grid(3, 8, (1, 1, 1), [0.0] * 3, [10.0] * 3, (0, 0, 0), O.WARP_SINE, 0.1)
+    law, form = product_scheme(rb, "eul_kg", 3)
+    q = initial_state(og, oracle_law("eul_kg", 3), "eul_kg", seed=9)
+    out = []
+    for flux in (rb.RusanovFlux(), rb.CentralFlux()):
+        dg = rb.DGSEM(law=law, grid=wrap_oracle_grid(og), volume_form=form, surface_numericalflux=flux,
+                      precision=precision)
+        assert dg.geometry == "curved" and dg.pipelined_ctas > 0
+        qg = rb.GridArray.from_numpy(q)
+        q_out = qg.similar()
+        dg.lsrk54_stage(qg, q_out, qg.similar(), 0, 0.0, 1e-3)
+        out.append(q_out.numpy())
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
