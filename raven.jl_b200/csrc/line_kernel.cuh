@@ -404,6 +404,9 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                     sm.aux.get((a < H0 ? own16 : far16) + (half ? -S16 : S16) * d,
                                (a < H0 ? own8 : far8) + (half ? -S8 : S8) * d, v);
             };
+            T scale[H0];  // metric and mass, formed in FP64 and rounded once
+#pragma unroll
+            for (int m = 0; m < H0; ++m) scale[m] = (T)(sm.geo[buf][DIR] * A.winv[m]);
             // ---- volume term
             T acc[H0][NS], o[H0][NAUX];
 #pragma unroll
@@ -544,17 +547,15 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 }
             }
             // reflection, metric and mass: the half counted from the far end has the sign turned
-            const double drdx = sm.geo[buf][DIR];
-            const T sc = half ? -(T)drdx : (T)drdx;
 #pragma unroll
             for (int m = 0; m < H0; ++m) {
-                const T scm = sc * (T)A.winv[m];
+                const T scm = half ? -scale[m] : scale[m];
 #pragma unroll
                 for (int s = 0; s < NS; ++s) acc[m][s] *= scm;
             }
             // ---- face term at the thread's first node: (wsJ nf) MJI with wsJ MJI = |drdx| / w_0
             {
-                const T fsc = (T)(fabs(drdx) * A.winv[0]);
+                const T fsc = fabs(scale[0]);
                 const T sn = half ? T(1) : T(-1);
                 // q- is the state itself, and its velocity and pressure are what the element across
                 // the face takes from it: both compute the same flux, and equal states (q+ is q- on

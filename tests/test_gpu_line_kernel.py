@@ -177,3 +177,36 @@ def test_curved_open_faces_have_no_jump(rb, cuda_ok, precision):
         dg.lsrk54_stage(qg, q_out, qg.similar(), 0, 0.0, 1e-3)
         out.append(q_out.numpy())
     assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nq", range(4, 9))
+def test_fp32_scale_is_rounded_once(rb, cuda_ok, nq):
+    """FP32 bulk: the factor of a line's sum, drdx / w, is formed in FP64 and rounded once.
+
+    A gas at rest without pressure but for one interior node, p = 2 (gamma = 2: p = rho e
+    exactly): along its x line the sum of a node is one product, 2 times a table entry, so
+    the momentum after a stage of unit weight is known to the bit.  (Central faces: the
+    wave speed of p = 0 is not taken.)"""
+    H0, a = (nq + 1) // 2, 1
+    f32 = np.float32
+    for K, L in (((3, 1, 1), 10.0), ((7, 1, 1), 10.0), ((5, 1, 1), 0.37), ((1, 1, 1), 1.7)):
+        og = O.Grid(3, nq, K, [0.0] * 3, [L, 1.0, 1.0], (1, 1, 1))
+        dg = rb.DGSEM(law=rb.EulerLaw(3, 2.0), grid=wrap_oracle_grid(og), volume_form=rb.WeakForm(),
+                      surface_numericalflux=rb.CentralFlux(), precision="fp32_bulk")
+        assert dg.pipelined_ctas > 0
+        q = np.zeros((og.np, 5, og.E), order="F")
+        q[:, 0, :] = 1.0
+        line = nq * (1 + nq) + np.arange(nq)  # j = k = 1
+        q[line[a], 4, :] = 2.0
+        qg = rb.GridArray.from_numpy(q)
+        q_out = qg.similar()
+        dg.lsrk_stage_range(qg, q_out, qg.similar(), 0.0, 1.0, 0, og.E, 0.0, 1.0)
+        got = q_out.numpy()[line, 1, 0]
+        _, w, D = og.lgl()
+        S, drdx = D * w[:, None], og.volume_metrics()[0, 0, 0]
+        for m in range(1, nq - 1):
+            far = m >= H0  # counted from the far end, with the sign turned
+            i, j = (nq - 1 - a, nq - 1 - m) if far else (a, m)
+            want = f32(f32(2) * f32(S[i, j])) * f32((-drdx if far else drdx) * (1.0 / w[j]))
+            if m != a:
+                assert got[m] == float(want), (K, L, m)
