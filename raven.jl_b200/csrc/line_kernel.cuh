@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 const int n = p0_node(h);
                 if (NP % NT != 0 && n >= NP) continue;
                 const T rho = (T)sm.q[buf][0][n];
-                const T rinv = rcp(rho);
+                const T rinv = rcp_inner(rho);
                 const T m0 = (T)sm.q[buf][1][n], m1 = (T)sm.q[buf][2][n], m2 = (T)sm.q[buf][3][n];
                 const T u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
                 const T rhoe = (T)sm.q[buf][4][n];
@@ -482,9 +482,10 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
                 auto two_point = [&](const T (&x)[NAUX], const T (&y)[NAUX], const T q, T (&F)[NS], auto exact) {
                     const T ua0 = (x[1] + y[1]) * T(0.5), ua1 = (x[2] + y[2]) * T(0.5), ua2 = (x[3] + y[3]) * T(0.5);
                     const T rs = x[0] + y[0], bs = x[4] + y[4];
-                    const T ir = rcp(rs), ib = rcp(bs);
+                    constexpr bool kExact = decltype(exact)::value;
+                    const T ir = newton_rcp<kExact>(rs), ib = newton_rcp<kExact>(bs);
                     T rlog, iblog;
-                    if constexpr (decltype(exact)::value) {
+                    if constexpr (kExact) {
                         rlog = log_mean(x[0], y[0], ir);
                         iblog = inverse_log_mean(x[4], y[4], ib);
                     } else {
@@ -564,13 +565,13 @@ __global__ void __launch_bounds__(line::Shape<Q>::TH, (line::min_ctas<T, Q>()))
 #pragma unroll
                 for (int s = 1; s < NS; ++s)
                     qm[s] = s == 4 && COMBO == EUL_WEAK ? o[0][4] : (T)sm.q[buf][s][end];
-                const T rm = qm[0] = COMBO == EUL_KG ? T(2) * o[0][0] : o[0][0], rmi = rcp(rm);
+                const T rm = qm[0] = COMBO == EUL_KG ? T(2) * o[0][0] : o[0][0], rmi = rcp_inner(rm);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) um[d] = COMBO == EUL_KG ? T(2) * o[0][1 + d] : o[0][1 + d];
                 if constexpr (COMBO == EUL_KG) pm = T(2) * o[0][5];
                 else if constexpr (COMBO == EUL_WEAK) pm = o[0][5];
                 else pm = pressure(rmi, qm[1], qm[2], qm[3], qm[4]);
-                const T rp = (T)tr[DIR][0], Ep = (T)tr[DIR][4], rinv = rcp(rp);
+                const T rp = (T)tr[DIR][0], Ep = (T)tr[DIR][4], rinv = rcp_inner(rp);
                 T mp[3], up[3];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {

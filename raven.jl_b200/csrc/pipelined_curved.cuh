@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const int n = (t & 31) + 32 * h + 128 * (t >> 5);
-            const T rho = (T)sm.q[0][n], rinv = rcp(rho);
+            const T rho = (T)sm.q[0][n], rinv = rcp_inner(rho);
             const T m0 = (T)sm.q[1][n], m1 = (T)sm.q[2][n], m2 = (T)sm.q[3][n], rhoe = (T)sm.q[4][n];
             const T u0 = m0 * rinv, u1 = m1 * rinv, u2 = m2 * rinv;
             const T p = pipec::gas<T>(A, 1) * (rhoe - (m0 * m0 + m1 * m1 + m2 * m2) * (T(0.5) * rinv));
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
             {
                 const T nv[3] = {(T)sg[0], (T)sg[1], (T)sg[2]}, wsJ = (T)sg[3];
                 const T rm = T(2) * o[0][0], pm = T(2) * o[0][5], Em = rm * (T(2) * o[0][4]);
-                const T rp = (T)tr[0], Ep = (T)tr[4], rinv = rcp(rp);
+                const T rp = (T)tr[0], Ep = (T)tr[4], rinv = rcp_inner(rp);
                 T um[3], mp[3], up[3], unm = T(0), unp = T(0);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(pipec::NT, 2) pipelined_curved_kernel(const __
                 }
                 const T pp = pipec::gas<T>(A, 1) * (Ep - (mp[0] * mp[0] + mp[1] * mp[1] + mp[2] * mp[2]) * (T(0.5) * rinv));
                 // the larger wave speed |u.n| + sqrt(gamma p / rho) (euler.jl:62-68)
-                const T wm = fabs(unm) + root(pipec::gas<T>(A, 0) * pm * rcp(rm));
+                const T wm = fabs(unm) + root(pipec::gas<T>(A, 0) * pm * rcp_inner(rm));
                 const T wp = fabs(unp) + root(pipec::gas<T>(A, 0) * pp * rinv);
                 // (q+ is q- on a boundary face: no jump, whatever the primitives' rounding)
                 const T mx = A.surface_rusanov && nbf >= 0 ? fmax(wm, wp) : T(0);

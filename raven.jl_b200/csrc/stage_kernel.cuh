@@ -318,7 +318,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
         } else {
             const T rho = q[0];
             const T rhoe = q[DIM + 1];
-            const T rinv = rcp(rho);
+            const T rinv = rcp_inner(rho);
             T u[DIM];
 #pragma unroll
             for (int d = 0; d < DIM; ++d) u[d] = q[1 + d] * rinv;
@@ -471,9 +471,10 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
                         const T b2 = aux[(DIM + 1) * NP + na];
                         const T uu2 = aux[(DIM + 2) * NP + na];
                         const T u2a = (own[DIM + 2] + uu2) * T(0.5);
-                        const T ir = rcp(own[0] + r2), ib = rcp(own[DIM + 1] + b2);
+                        constexpr bool kExact = decltype(exact)::value;
+                        const T ir = newton_rcp<kExact>(own[0] + r2), ib = newton_rcp<kExact>(own[DIM + 1] + b2);
                         T rlog, iblog;
-                        if constexpr (decltype(exact)::value) {
+                        if constexpr (kExact) {
                             rlog = log_mean(own[0], r2, ir);
                             iblog = inverse_log_mean(own[DIM + 1], b2, ib);
                         } else {
@@ -626,7 +627,7 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll
                 for (int side2 = 0; side2 < 2; ++side2) {
                     const T* qq = side2 == 0 ? q : qp;
-                    const T rho = qq[0], rhoe = qq[DIM + 1], rinv = rcp(rho);
+                    const T rho = qq[0], rhoe = qq[DIM + 1], rinv = rcp_inner(rho);
                     T u[DIM];
 #pragma unroll
                     for (int d = 0; d < DIM; ++d) u[d] = qq[1 + d] * rinv;

@@ -13,33 +13,57 @@
 namespace rb200 {
 
 // Reciprocal and square root by Newton's iteration from the hardware's approximations (PTX
-// rcp.approx and rsqrt.approx: some 20 bits in FP64, 23 in FP32), good to about a rounding.
-// The compiler's own divide and root branch to a slow path for extreme arguments, which cuts
-// the unrolled pair loops into blocks that cannot overlap; these do not branch.  Arguments
-// are densities, pressures and their like: normal and far from the ends of the range.
-__device__ __forceinline__ double rcp(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(y, fma(-x, y, 1.0), y);
-    return fma(y, fma(-x, y, 1.0), y);
+// rcp.approx and rsqrt.approx: some 20 bits in FP64, 23 in FP32).  The compiler's own divide and
+// root branch to a slow path for extreme arguments, which cuts the unrolled pair loops into
+// blocks that cannot overlap; these do not branch.  Within one unit in the last place for rcp of 2^-1022
+// .. 2^1022 in magnitude and root of 2^-960 .. 2^1022 (FP32: 2^-126 .. 2^126 and 2^-100 .. 2^126).
+// Beyond, 0, infinity, NaN and (root) negative arguments give what 1 / x and sqrt(x) give; a
+// subnormal argument counts as 0 (root returns it), and a subnormal reciprocal is 0.
+// rcp_inner leaves that test out, and makes NaN of 0 and infinity (with the test
+// everywhere entropy-conservative steps took 2 to 5 % longer, Kennedy-Gruber ones up to 2 %).  It is for
+// * densities: one of 0 or infinity makes the node's fluxes infinite or NaN either way;
+// * the pairs of the series path, where the NaN sends the line to the path with rcp.
+
+// whether an approximation is 0 or infinite: the argument is 0, infinite or at the ends of the
+// range, and Newton's iteration would make a NaN of it
+__device__ __forceinline__ bool at_end(double y) {
+    return ((((unsigned)__double2hiint(y) << 1) + 0x00200000u) & ~0x00200000u) == 0;
 }
-__device__ __forceinline__ float rcp(float x) {
+__device__ __forceinline__ bool at_end(float y) {
+    return (((__float_as_uint(y) << 1) + 0x01000000u) & ~0x01000000u) == 0;
+}
+template <bool ENDS>
+__device__ __forceinline__ double newton_rcp(double x) {
+    double y0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+    const double y = fma(y0, fma(-x, y0, 1.0), y0);
+    return ENDS && at_end(y0) ? y0 : fma(y, fma(-x, y, 1.0), y);
+}
+template <bool ENDS>
+__device__ __forceinline__ float newton_rcp(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
+    return ENDS && at_end(y) ? y : fmaf(y, fmaf(-x, y, 1.0f), y);
+}
+template <typename T>
+__device__ __forceinline__ T rcp(T x) {
+    return newton_rcp<true>(x);
+}
+template <typename T>
+__device__ __forceinline__ T rcp_inner(T x) {
+    return newton_rcp<false>(x);
 }
 __device__ __forceinline__ double root(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    y = fma(0.5 * y, fma(-(x * y), y, 1.0), y);
-    const double s = x * y;
-    return x == 0.0 ? x : fma(0.5 * y, fma(-s, s, x), s);
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+    const double y = fma(0.5 * y0, fma(-(x * y0), y0, 1.0), y0), s = x * y;
+    return at_end(y0) ? x : fma(0.5 * y, fma(-s, s, x), s);
 }
 __device__ __forceinline__ float root(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     const float s = x * y;
-    return x == 0.0f ? x : fmaf(0.5f * y, fmaf(-s, s, x), s);
+    return at_end(y) ? x : fmaf(0.5f * y, fmaf(-s, s, x), s);
 }
 
 // The logarithmic mean (a - b) / log(a / b) of logavg (numericalfluxes.jl:9-22) and its
