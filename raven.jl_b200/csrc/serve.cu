@@ -230,7 +230,9 @@ struct Class {
     // concurrently, so these overlap across classes) and DOF updates
     int64_t ticks_done = 0;
     double busy_ms = 0.0, dof_updates = 0.0;
-    double last_ms = 0.0;                        // device time of one of the last ticks
+    double last_ms = 0.0;                        // device time of one of the last ticks,
+    int64_t last_elems = 0;                      // which had this many elements
+    int64_t table_elems = 0;                     // elements in the table
     bool pipelined = false;                      // 3-D Nq=4, 6, 8 Euler KG or advection: the pipelined kernel
     int32_t* d_status = nullptr;                 // its bounded waits report here
     int active = 0;
@@ -511,7 +513,9 @@ cudaError_t admit(rb200_server* s) {
 // before the first solve finishes, up to some kBatchMs of device time, so that a class of
 // small solves does not wait for the host between its ticks (a tick of a few small solves
 // takes 30-60 us of the device, the host's poll as long again).  A request that arrives
-// meanwhile joins behind them.
+// meanwhile joins behind them.  The time of a tick is that of the last ones, in proportion to
+// the elements where there are more now: a large solve that joins a class of tiny ones gets
+// ticks of its own size, which the class's other solves, and requests, wait for one by one.
 //
 // A chunk is the work of one CTA at a time, so the table splits the running elements evenly:
 // about two chunks a CTA, of tile_elems to chunk_elems elements.  (At a fixed 8 tiles a 9^3
@@ -521,12 +525,14 @@ constexpr double kBatchMs = 0.25;
 constexpr int kMaxBatch = 16;
 cudaError_t launch_ticks(Class& c) {
     cudaError_t e = cudaSuccess;
+    const bool tuning = c.tune_done < 2 * c.ntiles;
     if (c.dirty) {
         int64_t total = 0;
         for (int i = 0; i < kMaxSolvesPerClass; ++i)
             if (c.slots[i]) total += c.h_solves[i].E;
-        const int64_t tiles = (total + 2 * (int64_t)c.grid * c.tile_elems - 1) / (2 * (int64_t)c.grid * c.tile_elems);
-        const int64_t len = std::min<int64_t>(std::max<int64_t>(tiles, 1) * c.tile_elems, c.chunk_elems);
+        const int64_t unit = c.tile_elems;
+        const int64_t tiles = (total + 2 * (int64_t)c.grid * unit - 1) / (2 * (int64_t)c.grid * unit);
+        const int64_t len = std::min<int64_t>(std::max<int64_t>(tiles, 1) * unit, c.chunk_elems);
         int n = 0;
         for (int i = 0; i < kMaxSolvesPerClass; ++i) {
             if (!c.slots[i]) continue;
@@ -535,6 +541,7 @@ cudaError_t launch_ticks(Class& c) {
                 c.h_chunks[n++] = Chunk{i, (int32_t)std::min<int64_t>(len, E - f), f};
         }
         c.table_chunks = n;
+        c.table_elems = total;
         e = cudaMemcpyAsync(c.d_solves, c.h_solves.data(), sizeof(SolveDesc) * kMaxSolvesPerClass,
                             cudaMemcpyHostToDevice, c.stream);
         if (e == cudaSuccess && n)
@@ -545,14 +552,14 @@ cudaError_t launch_ticks(Class& c) {
         c.dirty = false;
     }
     // autotuner: the first 2*ntiles ticks cycle through the tiles, then the fastest stays
-    const bool tuning = c.tune_done < 2 * c.ntiles;
     c.last_tile = tuning ? c.tune_done % c.ntiles : c.tile;
     int batch = 1;
     if (!tuning) {
         int64_t left = kMaxBatch;
         for (auto* sv : c.slots)
             if (sv) left = std::min<int64_t>(left, sv->req->nsteps - sv->steps_done);
-        const double ms = c.ticks_done > 0 ? c.last_ms : kBatchMs;
+        const double grown = (double)c.table_elems / (double)std::max<int64_t>(c.last_elems, 1);
+        const double ms = c.ticks_done > 0 ? c.last_ms * std::max(grown, 1.0) : kBatchMs;
         if (ms * left > kBatchMs) left = (int64_t)(kBatchMs / ms);
         batch = (int)std::max<int64_t>(left, 1);
     }
@@ -573,6 +580,7 @@ cudaError_t finish_ticks(rb200_server* s, Class& c) {
     float ms = 0;
     cudaEventElapsedTime(&ms, c.ev0, c.ev1);
     c.last_ms = ms / batch;
+    c.last_elems = c.table_elems;
     int64_t elems = 0;  // elements of the solves the ticks advanced
     for (auto* sv : c.slots)
         if (sv && sv->desc.start_tick <= done_tick) elems += sv->desc.E;

@@ -250,3 +250,30 @@ def test_ticks_enqueued_together(rb, S):
             tickets = [srv.submit(s) for s in specs]
             for t, ref in zip(tickets, alone):
                 assert np.array_equal(srv.wait(t)[0], ref)
+
+
+def test_large_solve_joins_a_class_of_tiny_ones(rb, S):
+    """Ticks are enqueued together by the time the next ones will take: a large solve that joins
+    a class whose ticks took some 30 us (eight and more at once) gets them one by one, so that
+    no batch of its ticks, of some milliseconds each, holds the class up.  Seen from the counts
+    of finished ticks, read more often than a tick of the large solve ends: batches of them
+    (four or more ticks between two reads) would show as ticks that took a millisecond each."""
+    import time
+
+    tiny, large = _spec(S, 3, 8, 1, (2, 2, 2), 40000), _spec(S, 3, 8, 1, (32, 32, 32), 20)
+    with S.Server(arena_bytes=3 << 30) as srv:
+        t0 = srv.submit(tiny)
+        while srv.class_stats() == [] or srv.class_stats()[0]["ticks"] < 100:
+            time.sleep(1e-3)
+        t1 = srv.submit(large)
+        assert srv.stats()["completed"] == 0
+        seen = []
+        while srv.stats()["completed"] == 0:
+            c = srv.class_stats()[0]
+            if not seen or c["ticks"] != seen[-1][0]:
+                seen.append((c["ticks"], c["device_ms"]))
+        steps = [(b[0] - a[0], b[1] - a[1]) for a, b in zip(seen, seen[1:])]
+        slow = [n for n, ms in steps if ms > n]  # a millisecond a tick and more: the large solve's
+        assert sum(slow) >= 10 and max(slow) < 4, steps
+        for t in (t0, t1):
+            assert np.isfinite(srv.wait(t)[0]).all()
