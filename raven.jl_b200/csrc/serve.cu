@@ -210,7 +210,6 @@ struct Class {
     std::vector<Chunk> h_chunks;
     std::vector<Solve*> slots;
     int chunk_elems = 1;                         // elements of a chunk at most; admission counts these
-    int tile_elems = 1;                          // and at least
     int grid = 1;                                // CTAs of the class's launches
     int nchunks = 0;                             // chunks of the running solves at chunk_elems each
     int32_t table_chunks = 0;                    // chunks in the table (upload source)
@@ -367,10 +366,7 @@ cudaError_t make_class(rb200_server* s, Class& c, const Req& r) {
         e = launch_batched(c.dim, c.nq, c.combo, c.prec, t, probe, 0, c.stream, &bps);
         if (e != cudaSuccess) return e;
         const int grid = std::max(1, bps) * nsm;  // fixed persistent grid
-        if (t == 1 || c.ntiles == 1) {
-            c.grid = grid;
-            c.tile_elems = c.epb[1];
-        }
+        if (t == 1 || c.ntiles == 1) c.grid = grid;
         cudaGraph_t g = nullptr;
         e = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
@@ -518,9 +514,10 @@ cudaError_t admit(rb200_server* s) {
 // ticks of its own size, which the class's other solves, and requests, wait for one by one.
 //
 // A chunk is the work of one CTA at a time, so the table splits the running elements evenly:
-// about two chunks a CTA, of tile_elems to chunk_elems elements.  (At a fixed 8 tiles a 9^3
-// solve at Nq = 8 gave 92 of 444 CTAs 8 elements each.)  A table so has at most the chunks
-// that admission counted plus two for each CTA and one for each solve.
+// about two chunks a CTA, of one tile to chunk_elems elements.  (At a fixed 8 tiles a 9^3
+// solve at Nq = 8 gave 92 of 444 CTAs 8 elements each.)  A chunk is whole tiles of the class's
+// choice, and of the largest candidate while the autotuner compares them.  A table so has at
+// most the chunks that admission counted plus two for each CTA and one for each solve.
 constexpr double kBatchMs = 0.25;
 constexpr int kMaxBatch = 16;
 cudaError_t launch_ticks(Class& c) {
@@ -530,15 +527,17 @@ cudaError_t launch_ticks(Class& c) {
         int64_t total = 0;
         for (int i = 0; i < kMaxSolvesPerClass; ++i)
             if (c.slots[i]) total += c.h_solves[i].E;
-        const int64_t unit = c.tile_elems;
+        const int64_t unit = c.pipelined ? 1 : c.epb[tuning ? c.ntiles - 1 : c.tile];
         const int64_t tiles = (total + 2 * (int64_t)c.grid * unit - 1) / (2 * (int64_t)c.grid * unit);
         const int64_t len = std::min<int64_t>(std::max<int64_t>(tiles, 1) * unit, c.chunk_elems);
         int n = 0;
         for (int i = 0; i < kMaxSolvesPerClass; ++i) {
             if (!c.slots[i]) continue;
             const int64_t E = c.h_solves[i].E;
-            for (int64_t f = 0; f < E && n < kMaxTableChunks; f += len)
+            for (int64_t f = 0; f < E; f += len) {
+                if (n == kMaxTableChunks) return cudaErrorInvalidConfiguration;  // not by the bound above
                 c.h_chunks[n++] = Chunk{i, (int32_t)std::min<int64_t>(len, E - f), f};
+            }
         }
         c.table_chunks = n;
         c.table_elems = total;
@@ -596,6 +595,7 @@ cudaError_t finish_ticks(rb200_server* s, Class& c) {
             for (int t = 1; t < c.ntiles; ++t)
                 if (c.tune_ms[t] / c.tune_n[t] < c.tune_ms[best] / c.tune_n[best]) best = t;
             c.tile = best;
+            c.dirty = true;  // chunks in whole tiles of the choice
         }
     }
     c.tick += batch;
