@@ -209,7 +209,9 @@ def test_snapshot_resume(rb, cuda_ok, precision, stepper):
 
 @pytest.mark.parametrize("ratio", [1.0, 1 + 1e-9, 1.01, 1.21, 1.23, 3.0])
 @pytest.mark.parametrize("dim,nq,sflux,precision", [(2, 5, "rusanov", "fp64"), (3, 4, "rusanov", "fp64"), (3, 5, "ec", "fp64"),
-                                                    (3, 8, "rusanov", "fp64"), (2, 4, "rusanov", "fp32_bulk")])
+                                                    (3, 8, "rusanov", "fp64"), (2, 4, "rusanov", "fp32_bulk"),
+                                                    (3, 5, "rusanov", "fp64"), (3, 6, "rusanov", "fp64"),
+                                                    (3, 7, "rusanov", "fp64")])
 def test_log_mean_branches(rb, cuda_ok, dim, nq, sflux, precision, ratio):
     """The entropy-conservative tendency of states whose density and rho/p take two values
     with a fixed ratio: equal values, values in the power series of the logarithmic mean and
@@ -218,6 +220,8 @@ def test_log_mean_branches(rb, cuda_ok, dim, nq, sflux, precision, ratio):
     2/h max_i sum_a |D[a,i] w_a/w_i - D[i,a]| max |flux| per field: 1e-12 in FP64, and 5e-6
     (some 40 roundings of 2^-24) in FP32 bulk."""
     og, dg, olaw, law = _build(rb, dim, nq, (3,) * dim, (1,) * dim, "eul_ec", O.WARP_NONE, sflux, precision)
+    # the half-line kernel, or (entropy surface flux, 2-D) the generic one
+    assert (dg.pipelined_ctas > 0) == (dim == 3 and sflux == "rusanov")
     rng = np.random.default_rng(5)
     shape = (og.np, og.E)
     rho = np.where(rng.random(shape) < 0.5, 1.0, ratio)

@@ -210,3 +210,51 @@ def test_fp32_scale_is_rounded_once(rb, cuda_ok, nq):
             want = f32(f32(2) * f32(S[i, j])) * f32((-drdx if far else drdx) * (1.0 / w[j]))
             if m != a:
                 assert got[m] == float(want), (K, L, m)
+
+
+@pytest.mark.parametrize("nq", range(4, 9))
+@pytest.mark.parametrize("scheme", SCHEMES)
+def test_fp32_bulk_steps(rb, cuda_ok, scheme, nq):
+    """Two FP32-bulk steps of every volume form on a grid with open faces."""
+    og, dg, olaw = _build(rb, nq, (3, 2, 3), (1, 0, 1), scheme, "fp32_bulk")
+    q = initial_state(og, olaw, scheme, seed=12)
+    qo, dqo = q.copy(order="F"), og.state(olaw)
+    for i in range(2):
+        og.lsrk54_step(olaw, qo, dqo, i * 1e-3, 1e-3)
+    qg = rb.GridArray.from_numpy(q)
+    rb.LSRK54(dg, qg, 1e-3).dostep(qg, 2)
+    dg.sync_status()
+    assert rel_err(qg.numpy(), qo) <= 1e-6
+
+
+@pytest.mark.parametrize("ratio", [1.21, 1.23, 3.0])
+@pytest.mark.parametrize("nq", range(4, 9))
+def test_log_mean_branches_in_steps(rb, cuda_ok, nq, ratio):
+    """One entropy-conservative step, both precisions, of a state whose density and rho/p take
+    two values: on either side of the end of the logarithmic means' series (a ratio of 1.222)
+    and far beyond, so that lines take their sums again with the logarithms.
+
+    The step is short: in FP32 bulk the register's error, 5e-6 of its terms' size (some 100 here,
+    see test_log_mean_branches), times 1e-4 is 1e-7 of the state; a mean that is wrong by
+    1e-3 would change it by 1e-5."""
+    og, dg, olaw = _build(rb, nq, (3, 2, 2), (1, 0, 1), "eul_ec")
+    rng = np.random.default_rng(13)
+    shape = (og.np, og.E)
+    rho = np.where(rng.random(shape) < 0.5, 1.0, ratio)
+    p = rho / np.where(rng.random(shape) < 0.5, 1.1, 1.1 * ratio)
+    u = (0.4, -0.3, 0.2)
+    E = p / 0.4 + rho * sum(v * v for v in u) / 2
+    q = np.asfortranarray(np.stack([rho] + [rho * v for v in u] + [E], axis=1))
+    dt = 1e-4
+    qo, dqo = q.copy(order="F"), og.state(olaw)
+    og.lsrk54_step(olaw, qo, dqo, 0.0, dt)
+    qg = rb.GridArray.from_numpy(q)
+    s = rb.LSRK54(dg, qg, dt)
+    s.dostep(qg, 1)
+    dg.sync_status()
+    assert rel_err(qg.numpy(), qo) <= 1e-12 and rel_err(s.dq.numpy(), dqo) <= 1e-11
+    _, dg32, _ = _build(rb, nq, (3, 2, 2), (1, 0, 1), "eul_ec", "fp32_bulk")
+    qg = rb.GridArray.from_numpy(q)
+    rb.LSRK54(dg32, qg, dt).dostep(qg, 1)
+    dg32.sync_status()
+    assert rel_err(qg.numpy(), qo) <= 1e-6
