@@ -27,7 +27,7 @@ struct PipeArgs {
     int64_t e_begin;
     int32_t mode;
     int32_t surface_rusanov;
-    double rka, rkb_dt, gamma;
+    double rka, rkb_dt;
     double S[64];    // the volume term's table, entry a*Nq + id: see pipe_tables
     double w[8];
     double winv[8];  // 1 / w
@@ -46,7 +46,6 @@ struct PipeArgs {
 // Returns whether the half-line kernel's reading of the Euler tables holds: w even and the
 // table odd under reflection of the line, to 8 roundings (every Lobatto line's are).
 inline bool pipe_tables(PipeArgs& p, int combo, int nq, double gamma, const double* D, const double* w) {
-    p.gamma = gamma;
     p.gas[0] = gamma, p.gas[1] = gamma - 1.0, p.gas[2] = 1.0 / (2.0 * (gamma - 1.0));
     for (int i = 0; i < 3; ++i) p.gasf[i] = (float)p.gas[i];
     for (int i = 0; i < nq; ++i) {
@@ -115,9 +114,8 @@ struct ElemRef {
 
 namespace pipe {
 
-constexpr int NQ = 8, NP = 512, NS = 5, NAUX = 6, NSLOT = 384;  // the Nq = 8 element
-constexpr int PAD(int n) { return n + (n >> 3); }  // one vector slot of padding every 8 nodes
-constexpr int NPP = PAD(NP);                       // padded plane length
+constexpr int NS = 5, NAUX = 6;                    // fields and partner values of a node (Euler)
+constexpr int PAD(int n) { return n + (n >> 3); }  // one slot of padding every 8 nodes
 
 // Sizes of an element with Q nodes per direction (Q even: an element's state is then a
 // whole number of 16-byte units, as the bulk copies need).
@@ -166,9 +164,6 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
