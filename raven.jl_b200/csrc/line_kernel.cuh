@@ -13,22 +13,24 @@
 // which it loads into registers before its pairs: there is no face buffer and no face phase.
 // Sums pass from one direction's threads to the next's through shared memory.
 //
-// The kernel before it gave each node its full lines of partners: 4.2 K shared-memory load
-// wavefronts an element (Nq = 8, FP64) and 13 K warp instructions; here 2.5 K and 9.2 K.
+// The kernels before it gave each node its full lines of partners: 3.4 K shared-memory load
+// wavefronts an element (Nq = 8; FP32 2.8 K) and 11.9 K warp instructions (13.5 K); here 2.3 K (1.4 K)
+// and 9.7 K (9.3 K).
 //
-// What bounds it (Nq = 8): an element takes an SM 5.8 K cycles in FP64 and 4.0 K in FP32 bulk,
-// whether its state comes from HBM or from L2, and with 2 or 3 CTAs an SM.  No unit is full
-// (FP64: the FP64 pipe 50 %, issue 40 %, the L1 data pipe 52 %; FP32: issue 60 %): with 8 or
-// 12 warps an SM the latencies of shared memory, the FP64 pipe and the two barriers are not
-// covered.  The limits above are 2.9 K cycles (FP64 pipe) and 3.5 K (HBM, 152 B/node).
-// Measured on B200, one LSRK(5,4) step, before -> after: Kennedy-Gruber Nq = 8, 32^3 FP64 4607
-// -> 3712 us, FP32 bulk 3515 -> 2571; Nq = 6, 24^3 864 -> 712 and 690 -> 538; Nq = 4, 30^3 449
-// -> 368 and 411 -> 274; entropy conservative Nq = 5, 18^3 FP64 914 -> 379 and weak form Nq = 7,
-// 15^3 FP64 1135 -> 325 (both from the generic kernel).
-// Tried and slower: one state buffer with the old state read again at the end (3 CTAs an SM at
-// 168 registers, spills: 4107-4800); a fifth warp that only fetches (168 registers at 2
-// CTAs); the traces one element ahead (3800); the register added at the end from a buffer
-// of its own (4317).
+// What bounds it (Nq = 8): an element takes an SM 3.3 us in FP64 and 2.15 us in FP32 bulk (6.4 K and
+// 4.2 K cycles), from 16^3 elements to 32^3.  No unit is full (FP64: the FP64 pipe 47 %, issue 39 %, the
+// L1 data pipe 54 %; FP32: issue 59 %): with 8 or 12 warps an SM the latencies of shared memory, the
+// FP64 pipe and the two barriers are not covered.  The FP64 pipe alone would
+// take 2.9 K cycles, HBM 3.5 K (152 B/node).
+// Measured on B200, one LSRK(5,4) step, the kernels before -> this one: Kennedy-Gruber Nq = 8, 32^3,
+// over three states in turn FP64 4667 -> 4060 us, FP32 bulk 3562 -> 2740 (on one state again and again
+// 3.52-3.70 ms and 2.35-2.41); Nq = 6, 24^3 864 -> 712 and 690 -> 538; Nq = 4, 30^3 449 -> 368 and 411 ->
+// 274; entropy conservative Nq = 5, 18^3 FP64 914 -> 379 and weak form Nq = 7, 15^3 FP64 1135 -> 330
+// (both from the generic kernel).
+// Tried and slower, in us a step at Nq = 8, 32^3 FP64 on one state, against 3712 then: one state
+// buffer with the old state read again at the end (3 CTAs an SM at 168 registers, spills: 4107-4800);
+// the traces one element ahead (3800); the register added at the end from a buffer of its own
+// (4317).  A fifth warp that only fetches would leave 168 registers at 2 CTAs: not tried.
 //
 // Nq = 8: z, then y, then x lines.  A warp owns two z planes in the y and x phases and when it
 // builds the partner values, so those hand-overs need no CTA barrier; two barriers an element.
@@ -100,7 +102,7 @@ struct Smem {
 };
 
 // CTAs per SM the registers are sized for, FP64 and FP32.  A thread holds its half line, its sums
-// and three traces: 254 registers in FP64 at Nq = 8, 164 in FP32; one CTA more an SM spills and
+// and three traces: 254 registers in FP64 at Nq = 8, 168 in FP32; one CTA more an SM spills and
 // is slower (Nq = 8 FP64 3 CTAs 1108 against 955 us at 20^3, FP32 4 CTAs 693 against 622; Nq = 6,
 // 24^3: 5 and 7 CTAs 752 and 603 against 712 and 538).
 #ifndef RB200_LINE_MIN8

@@ -18,9 +18,9 @@
 // What bounds it: HBM (256 B/node in FP64, 220 in FP32 bulk: 6.0 and 5.1 K cycles an element and
 // SM at the measured peak) and, in FP64, the FP64 pipe (4.5 K).  The kernels before this one (256
 // threads, each node its full lines of partners with their metric rows) took 16.5 and 12.2 K, and
-// this one 12.2 and 8.4 K: B200, one LSRK(5,4) step, FP64 13^3 635 -> 468 us, FP32 bulk 16^3 883 ->
-// 602.  Two CTAs of 128 threads share an SM (255 registers a thread in FP64; shared memory 107
-// and 83 KB a CTA): 8 warps do not cover the latencies between the two barriers.
+// this one 12.2 and 8.4 K: B200, one LSRK(5,4) step, FP64 13^3 635 -> 475 us, FP32 bulk 16^3 883 ->
+// 606.  Two CTAs of 128 threads share an SM (255 registers a thread in FP64; shared memory 110
+// and 85 KB a CTA): 8 warps do not cover the latencies between the two barriers.
 //
 // Every mbarrier wait is bounded: on expiry the CTA records RB200 status TIMEOUT and returns.
 #pragma once

@@ -404,7 +404,9 @@ __device__ __forceinline__ void stage_element(const StageArgs& A, const ElemPtrs
 #pragma unroll kUnroll
             for (int a = 0; a < NQ; ++a) {
                 const int na = base + a * stride;
-                // D[a, id]: from shared memory, but 3-D FP64 from the parameters (each measured faster)
+                // D[a, id]: from shared memory, but 3-D FP64 from the parameters (each measured faster; as
+                // parameters 2-D FP64 at 100^2, N = 7 took 246 us a step for KG and 191 for the weak form,
+                // here 204 and 179; N = 3 to 4 gain 0 to 4 %)
                 const T Dai = kSharedD ? sD[a + NQ * idd] : (T)A.D[a + NQ * idd];
                 if constexpr (COMBO == ADV_WEAK) {
                     acc[0] += Dai * aux[dir * NP + na];
